@@ -698,6 +698,12 @@ enum : uint32_t {
 // Postfix interpreter over the ops [pc0, pc1) of DeProgram.ops (generic graphs) in
 // one of the SF_EVAL_* modes; the whole program is [0, n_ops). Inlined into the two
 // entry points below, so the whole-program one keeps its constant range and modes.
+//
+// The lanes of a call run the lowest op any of them stands at; the others wait there.
+// Lanes that skip a bounded branch, leave a loop early or search other copies meet
+// again at the op where their ways join, so every op is issued once for all the lanes
+// that need it. With one program counter per lane, lanes a few ops apart stayed apart
+// to the end of the program and each op was issued once for every such group.
 __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t mode, uint32_t pc0, uint32_t pc1) {
     const bool exact = mode == SF_EVAL_EXACT, probe = mode == SF_EVAL_PROBE;
     // the copy searches in flight, one per nesting level (eval.rs:808 recurses into the
@@ -714,8 +720,13 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
     int sp = 0;
     float3 seed_p = c;
     float seed_dr = 1.0f;
-    for (uint32_t pc = pc0; pc < pc1; ++pc) {
-        const DeOp& op = P.ops[pc];
+    const uint32_t lanes = __activemask();
+    uint32_t pc = pc0;
+    for (;;) {
+        const uint32_t at = __reduce_min_sync(lanes, pc < pc1 ? pc : 0xffffffffu);
+        if (at == 0xffffffffu) break;
+        if (pc != at) continue;
+        const DeOp& op = P.ops[at];
         switch (op.code) {
         case SF_OP_BEGIN:
             s.p = c; s.dr = 1.0f; s.iter = 0; s.t0 = s.t1 = s.t2 = s.t3 = SF_INF;
@@ -845,6 +856,7 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
             }
             break;
         }
+        ++pc;
     }
     return sp > 0 ? stack[sp - 1] : raw_empty();
 }
