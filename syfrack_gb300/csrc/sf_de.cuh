@@ -723,9 +723,11 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
     const uint32_t lanes = __activemask();
     uint32_t pc = pc0;
     for (;;) {
-        const uint32_t at = __reduce_min_sync(lanes, pc < pc1 ? pc : 0xffffffffu);
+        // a lane past its own range stands nowhere: another's range may start there
+        const uint32_t here = pc < pc1 ? pc : 0xffffffffu;
+        const uint32_t at = __reduce_min_sync(lanes, here);
         if (at == 0xffffffffu) break;
-        if (pc != at) continue;
+        if (here != at) continue;
         const DeOp& op = P.ops[at];
         switch (op.code) {
         case SF_OP_BEGIN:
