@@ -89,18 +89,27 @@ __device__ __forceinline__ DeSampleF de_finalize(const DeProgram& P, const DeRaw
     return s;
 }
 
-// measure (eval.rs:299-331).
-__device__ __forceinline__ float trap_measure(uint32_t m, float3 p) {
+// measure (eval.rs:299-331). The angles and the logarithm stay out of line: inlined
+// into the interpreter and every form, their code crowds the instruction cache.
+static __device__ __noinline__ float trap_measure_rare(uint32_t m, float3 p) {
     const float TAU = 6.2831855f;
     switch (m) {
-    case SF_MEASURE_AXIS_X: return sqrtf(p.y * p.y + p.z * p.z);
-    case SF_MEASURE_AXIS_Y: return sqrtf(p.x * p.x + p.z * p.z);
-    case SF_MEASURE_AXIS_Z: return sqrtf(p.x * p.x + p.y * p.y);
-    case SF_MEASURE_PLANE_Y: return fabsf(p.y);
     case SF_MEASURE_ANGLE_XY: return (p.x == 0.f && p.y == 0.f) ? 0.5f : atan2f(p.y, p.x) / TAU + 0.5f;
     case SF_MEASURE_ANGLE_XZ: return (p.x == 0.f && p.z == 0.f) ? 0.5f : atan2f(p.z, p.x) / TAU + 0.5f;
     case SF_MEASURE_ANGLE_YZ: return (p.y == 0.f && p.z == 0.f) ? 0.5f : atan2f(p.z, p.y) / TAU + 0.5f;
-    case SF_MEASURE_LOG_NORM: return log1pf(len3(p));
+    default: return log1pf(len3(p));
+    }
+}
+__device__ __forceinline__ float trap_measure(uint32_t m, float3 p) {
+    switch (m) {
+    case SF_MEASURE_AXIS_X: return sqrtf(fmaf(p.z, p.z, p.y * p.y));
+    case SF_MEASURE_AXIS_Y: return sqrtf(fmaf(p.z, p.z, p.x * p.x));
+    case SF_MEASURE_AXIS_Z: return sqrtf(fmaf(p.y, p.y, p.x * p.x));
+    case SF_MEASURE_PLANE_Y: return fabsf(p.y);
+    case SF_MEASURE_ANGLE_XY:
+    case SF_MEASURE_ANGLE_XZ:
+    case SF_MEASURE_ANGLE_YZ:
+    case SF_MEASURE_LOG_NORM: return trap_measure_rare(m, p);
     default: return len3(p);
     }
 }
@@ -206,8 +215,27 @@ __device__ __forceinline__ void spherical_power(float3 p, float r, uint32_t n, f
     deriv = float(n) * prev;
 }
 
-// Power node (eval.rs:456-476), including the trigonometric path for
-// non-integer exponents and radii below 1e-12.
+// The Power node's trigonometric path (non-integer exponents, radii below 1e-12): the
+// unit direction, its radius and the factor of dr.
+struct PowerTrig {
+    float3 dir;
+    float zr, factor;
+};
+__device__ __forceinline__ PowerTrig power_trig(float3 p, float radius, float power) {
+    PowerTrig o;
+    float r = fmaxf(radius, 1e-12f);
+    float theta = radius >= 1e-12f ? atan2f(sqrtf(fmaf(p.x, p.x, p.y * p.y)), p.z)
+                                   : acosf(fminf(fmaxf(p.z / r, -1.0f), 1.0f));
+    float phi = atan2f(p.y, p.x);
+    o.factor = powf(r, power - 1.0f) * power;
+    o.zr = powf(r, power);
+    float st, ct, sp, cp;
+    sincosf(theta * power, &st, &ct);
+    sincosf(phi * power, &sp, &cp);
+    o.dir = mk3(st * cp, st * sp, ct);
+    return o;
+}
+// Power node (eval.rs:456-476).
 __device__ __forceinline__ void power_op(float3& p, float& dr, float radius, float power, uint32_t power_int) {
     if (radius >= 1e-12f && power_int != 0) {
         float3 q;
@@ -217,16 +245,9 @@ __device__ __forceinline__ void power_op(float3& p, float& dr, float radius, flo
         dr *= dv;
         return;
     }
-    float r = fmaxf(radius, 1e-12f);
-    float theta = radius >= 1e-12f ? atan2f(sqrtf(p.x * p.x + p.y * p.y), p.z)
-                                   : acosf(fminf(fmaxf(p.z / r, -1.0f), 1.0f));
-    float phi = atan2f(p.y, p.x);
-    dr *= powf(r, power - 1.0f) * power;
-    float zr = powf(r, power);
-    float st, ct, sp, cp;
-    sincosf(theta * power, &st, &ct);
-    sincosf(phi * power, &sp, &cp);
-    p = mk3(st * cp, st * sp, ct) * zr;
+    const PowerTrig q = power_trig(p, radius, power);
+    dr *= q.factor;
+    p = q.dir * q.zr;
 }
 
 __device__ __forceinline__ float bulb_fence(float3 p, float dr) {
@@ -390,6 +411,15 @@ struct PState {
     float t0, t1, t2, t3;
 };
 
+// Euler rotation by the cosines and sines of the z, y and x angles, prepared once per
+// program. The fused products are written out (the cosine's in every sum): this is the
+// contraction the compiler picks for rotate_euler_xyz below.
+__device__ __forceinline__ float3 rotate_prepared(float3 p, const float* r) {
+    const float cz = r[0], sz = r[1], cy = r[2], sy = r[3], cx = r[4], sx = r[5];
+    float3 q = mk3(fmaf(cz, p.x, -(sz * p.y)), fmaf(cz, p.y, sz * p.x), p.z);
+    q = mk3(fmaf(cy, q.x, sy * q.z), q.y, fmaf(cy, q.z, -(sy * q.x)));
+    return mk3(q.x, fmaf(cx, q.y, -(sx * q.z)), fmaf(cx, q.z, sx * q.y));
+}
 __device__ __forceinline__ float3 rotate_euler_xyz(float3 p, float3 a) {
     float3 q = p;
     q = mk3(cosf(a.z) * q.x - sinf(a.z) * q.y, sinf(a.z) * q.x + cosf(a.z) * q.y, q.z);
@@ -399,6 +429,40 @@ __device__ __forceinline__ float3 rotate_euler_xyz(float3 p, float3 a) {
 }
 __device__ __forceinline__ float to_rad(float d) { return d * (3.14159265358979323846f / 180.0f); }
 
+// Constants that depend on an op's parameters alone, computed once when a program is
+// uploaded (k_prepare_program) by the same device functions an evaluation would call,
+// so every sample keeps its bits. Evaluated per sample, a Rotate's six sines and
+// cosines were its whole cost and most of the interpreter's executed code, whose
+// instruction-cache misses were 66% of the trace kernel's stalls on generic graphs.
+//   Rotate          f[2..7] = cos z, sin z, cos y, sin y, cos x, sin x (the angles are not kept)
+//   Mirror, Plane   f[4..6] = the unit normal
+//   SphereFold      f[2..4] = min radius^2, fixed radius^2, their quotient
+//   Kaleido         f[1] = sector
+__device__ __forceinline__ void prepare_op(DeOp& op) {
+    switch (op.code) {
+    case SF_NODE_ROTATE: {
+        const float ax = to_rad(op.f[0]), ay = to_rad(op.f[1]), az = to_rad(op.f[2]);
+        op.f[2] = cosf(az); op.f[3] = sinf(az);
+        op.f[4] = cosf(ay); op.f[5] = sinf(ay);
+        op.f[6] = cosf(ax); op.f[7] = sinf(ax);
+        break;
+    }
+    case SF_NODE_MIRROR:
+    case SF_NODE_PLANE: {
+        const float3 n = safe_normalize3(ld3(op.f));
+        op.f[4] = n.x; op.f[5] = n.y; op.f[6] = n.z;
+        break;
+    }
+    case SF_NODE_SPHERE_FOLD: {
+        const float mr2 = op.f[0] * op.f[0], fr2 = op.f[1] * op.f[1];
+        op.f[2] = mr2; op.f[3] = fr2; op.f[4] = fr2 / mr2;
+        break;
+    }
+    case SF_NODE_KALEIDO: op.f[1] = 6.2831855f / float(op.a > 0 ? op.a : 1u); break;
+    default: break;
+    }
+}
+
 __device__ __forceinline__ float terrain_hash(int cx, int cy, int cz, uint32_t seed) {
     uint32_t h = (uint32_t(cx) * 0x8da6b343u) ^ (uint32_t(cy) * 0xd8163841u) ^ (uint32_t(cz) * 0xcb1ab31fu) ^ seed;
     h = (h ^ (h >> 16)) * 0x7feb352du;
@@ -406,7 +470,7 @@ __device__ __forceinline__ float terrain_hash(int cx, int cy, int cz, uint32_t s
     h ^= h >> 16;
     return float(h >> 8) / 16777216.0f;
 }
-static __device__ float terrain_noise(float3 p, uint32_t seed) {
+static __device__ __noinline__ float terrain_noise(float3 p, uint32_t seed) {
     float3 base = mk3(floorf(p.x), floorf(p.y), floorf(p.z));
     float3 f = p - base;
     float3 t = f * f * (mk3(3.f, 3.f, 3.f) - f * 2.0f);
@@ -421,14 +485,59 @@ static __device__ float terrain_noise(float3 p, uint32_t seed) {
     return r;
 }
 
+// Point ops with angles or remainders, out of line like trap_measure_rare: they change
+// the point alone.
+static __device__ __noinline__ float3 bend_point(const DeOp& op, float3 p) {
+    switch (op.code) {
+    case SF_NODE_KALEIDO: {
+        float sector = op.f[1];
+        float a = atan2f(p.z, p.x) + to_rad(op.f[0]);
+        a = fabsf(rem_euclid(a + sector * 0.5f, sector) - sector * 0.5f);
+        float r = sqrtf(fmaf(p.z, p.z, p.x * p.x));
+        float sn, cs;
+        sincosf(a, &sn, &cs);
+        p.x = r * cs; p.z = r * sn;
+        return p;
+    }
+    case SF_NODE_TWIST: {
+        float sn, cs; sincosf(op.f[0] * p.y, &sn, &cs);
+        float x = diff_of_products(cs, p.x, sn, p.z), z = sum_of_products(sn, p.x, cs, p.z);
+        p.x = x; p.z = z;
+        return p;
+    }
+    case SF_NODE_BEND: {
+        float sn, cs; sincosf(op.f[0] * p.x, &sn, &cs);
+        float x = diff_of_products(cs, p.x, sn, p.y), y = sum_of_products(sn, p.x, cs, p.y);
+        p.x = x; p.y = y;
+        return p;
+    }
+    case SF_NODE_TILE: {
+        float3 per = ld3(op.f), h = per * 0.5f;
+        p = mk3(rem_euclid(p.x + h.x, per.x) - h.x, rem_euclid(p.y + h.y, per.y) - h.y,
+                  rem_euclid(p.z + h.z, per.z) - h.z);
+        return p;
+    }
+    case SF_NODE_REPEAT_FINITE: {
+        float3 per = ld3(op.f);
+        float3 last = mk3(float(op.a) - 1.0f, float(op.b) - 1.0f, float(op.c) - 1.0f);
+        float3 h = last * 0.5f;
+        float3 q = p / per + h + mk3(0.5f, 0.5f, 0.5f);
+        float3 cell = mk3(fminf(fmaxf(floorf(q.x), 0.f), last.x), fminf(fmaxf(floorf(q.y), 0.f), last.y),
+                          fminf(fmaxf(floorf(q.z), 0.f), last.z)) - h;
+        p = p - cell * per;
+        return p;
+    }
+    default: return p;
+    }
+}
 static __device__ void apply_point_op(const DeOp& op, PState& s, float3 c, float3 seed_p, float seed_dr) {
     switch (op.code) {
     case SF_NODE_TRANSLATE: s.p = s.p + ld3(op.f); break;
-    case SF_NODE_ROTATE: s.p = rotate_euler_xyz(s.p, mk3(to_rad(op.f[0]), to_rad(op.f[1]), to_rad(op.f[2]))); break;
+    case SF_NODE_ROTATE: s.p = rotate_prepared(s.p, op.f + 2); break;
     case SF_NODE_SCALE: s.p = s.p * op.f[0]; s.dr *= fabsf(op.f[0]); break;
     case SF_NODE_SCALE_AXES: { float3 f = ld3(op.f); s.p = s.p * f; s.dr *= max3(f); break; }
     case SF_NODE_MIRROR: {
-        float3 nn = safe_normalize3(ld3(op.f));
+        float3 nn = ld3(op.f + 4);
         float h = dot3(s.p, nn) - op.f[3];
         if (h < 0.0f) s.p = s.p - nn * (2.0f * h);
         break;
@@ -449,8 +558,8 @@ static __device__ void apply_point_op(const DeOp& op, PState& s, float3 c, float
     }
     case SF_NODE_SPHERE_FOLD: {
         float r2 = dot3(s.p, s.p);
-        float mr2 = op.f[0] * op.f[0], fr2 = op.f[1] * op.f[1];
-        float k = r2 < mr2 ? fr2 / mr2 : (r2 < fr2 ? fr2 / r2 : 1.0f);
+        float mr2 = op.f[2], fr2 = op.f[3];
+        float k = r2 < mr2 ? op.f[4] : (r2 < fr2 ? fr2 / r2 : 1.0f);
         s.p = s.p * k; s.dr *= k;
         break;
     }
@@ -471,16 +580,6 @@ static __device__ void apply_point_op(const DeOp& op, PState& s, float3 c, float
         s.p = z; s.dr *= sc;
         break;
     }
-    case SF_NODE_KALEIDO: {
-        float sector = 6.2831855f / float(op.a > 0 ? op.a : 1u);
-        float a = atan2f(s.p.z, s.p.x) + to_rad(op.f[0]);
-        a = fabsf(rem_euclid(a + sector * 0.5f, sector) - sector * 0.5f);
-        float r = sqrtf(s.p.x * s.p.x + s.p.z * s.p.z);
-        float sn, cs;
-        sincosf(a, &sn, &cs);
-        s.p.x = r * cs; s.p.z = r * sn;
-        break;
-    }
     case SF_NODE_POWER: power_op(s.p, s.dr, len3(s.p), op.f[0], op.a); break;
     case SF_NODE_ADD_ORIGIN: s.p = s.p + c; s.dr += 1.0f; break;
     case SF_NODE_ADD_SEED: { float3 m = ld3(op.f); s.p = s.p + seed_p * m; s.dr += seed_dr * max3(abs3(m)); break; }
@@ -490,34 +589,9 @@ static __device__ void apply_point_op(const DeOp& op, PState& s, float3 c, float
         s.dr += max3(abs3(m));
         break;
     }
-    case SF_NODE_TWIST: {
-        float sn, cs; sincosf(op.f[0] * s.p.y, &sn, &cs);
-        float x = cs * s.p.x - sn * s.p.z, z = sn * s.p.x + cs * s.p.z;
-        s.p.x = x; s.p.z = z;
+    case SF_NODE_KALEIDO: case SF_NODE_TWIST: case SF_NODE_BEND: case SF_NODE_TILE: case SF_NODE_REPEAT_FINITE:
+        s.p = bend_point(op, s.p);
         break;
-    }
-    case SF_NODE_BEND: {
-        float sn, cs; sincosf(op.f[0] * s.p.x, &sn, &cs);
-        float x = cs * s.p.x - sn * s.p.y, y = sn * s.p.x + cs * s.p.y;
-        s.p.x = x; s.p.y = y;
-        break;
-    }
-    case SF_NODE_TILE: {
-        float3 per = ld3(op.f), h = per * 0.5f;
-        s.p = mk3(rem_euclid(s.p.x + h.x, per.x) - h.x, rem_euclid(s.p.y + h.y, per.y) - h.y,
-                  rem_euclid(s.p.z + h.z, per.z) - h.z);
-        break;
-    }
-    case SF_NODE_REPEAT_FINITE: {
-        float3 per = ld3(op.f);
-        float3 last = mk3(float(op.a) - 1.0f, float(op.b) - 1.0f, float(op.c) - 1.0f);
-        float3 h = last * 0.5f;
-        float3 q = s.p / per + h + mk3(0.5f, 0.5f, 0.5f);
-        float3 cell = mk3(fminf(fmaxf(floorf(q.x), 0.f), last.x), fminf(fmaxf(floorf(q.y), 0.f), last.y),
-                          fminf(fmaxf(floorf(q.z), 0.f), last.z)) - h;
-        s.p = s.p - cell * per;
-        break;
-    }
     case SF_NODE_TRAP: {
         float v = trap_measure(op.b, s.p);
         DeRaw tmp;
@@ -530,18 +604,21 @@ static __device__ void apply_point_op(const DeOp& op, PState& s, float3 c, float
     }
 }
 
+// x / dr; dr is exactly 1 on every chain that does not scale, and x / 1 is x.
+__device__ __forceinline__ float over_dr(float x, float dr) { return dr == 1.0f ? x : x / dr; }
+
 // fence (eval.rs:558-599).
 static __device__ float fence_op(const DeOp& op, const PState& s) {
     switch (op.code) {
-    case SF_NODE_SPHERE: return (len3(s.p) - op.f[0]) / s.dr;
+    case SF_NODE_SPHERE: return over_dr(len3(s.p) - op.f[0], s.dr);
     case SF_NODE_TORUS: {
-        float q = sqrtf(s.p.x * s.p.x + s.p.z * s.p.z) - op.f[0];
-        return (sqrtf(q * q + s.p.y * s.p.y) - op.f[1]) / s.dr;
+        float q = sqrtf(fmaf(s.p.z, s.p.z, s.p.x * s.p.x)) - op.f[0];
+        return over_dr(sqrtf(fmaf(s.p.y, s.p.y, q * q)) - op.f[1], s.dr);
     }
     case SF_NODE_CYLINDER: {
-        float qx = sqrtf(s.p.x * s.p.x + s.p.z * s.p.z) - op.f[0], qy = fabsf(s.p.y) - op.f[1];
+        float qx = sqrtf(fmaf(s.p.z, s.p.z, s.p.x * s.p.x)) - op.f[0], qy = fabsf(s.p.y) - op.f[1];
         float mx = fmaxf(qx, 0.f), my = fmaxf(qy, 0.f);
-        return (sqrtf(mx * mx + my * my) + fminf(fmaxf(qx, qy), 0.0f)) / s.dr;
+        return over_dr(sqrtf(fmaf(mx, mx, my * my)) + fminf(fmaxf(qx, qy), 0.0f), s.dr);
     }
     case SF_NODE_BOX: return box_fence(s.p, ld3(op.f), s.dr);
     case SF_NODE_ROUND_BOX: {
@@ -549,7 +626,7 @@ static __device__ float fence_op(const DeOp& op, const PState& s) {
         float r = fminf(op.f[3], min3(half));
         float3 q = abs3(s.p) - (half - mk3(r, r, r));
         float3 qm = mk3(fmaxf(q.x, 0.f), fmaxf(q.y, 0.f), fmaxf(q.z, 0.f));
-        return (len3(qm) + fminf(max3(q), 0.0f) - r) / s.dr;
+        return over_dr(len3(qm) + fminf(max3(q), 0.0f) - r, s.dr);
     }
     case SF_NODE_ROCK: {
         float3 half = ld3(op.f);
@@ -560,8 +637,8 @@ static __device__ float fence_op(const DeOp& op, const PState& s) {
                        0.14f * terrain_noise(q * 4.17f, op.a + 193u) - 0.5f;
         return ((len3(s.p / half) - 1.0f - e * relief) * h / (1.0f + 5.22f * e)) / s.dr;
     }
-    case SF_NODE_PLANE: return (dot3(s.p, safe_normalize3(ld3(op.f))) - op.f[3]) / s.dr;
-    case SF_NODE_NORM_FENCE: return (len3(s.p) - op.f[0]) / fabsf(s.dr);
+    case SF_NODE_PLANE: return over_dr(dot3(s.p, ld3(op.f + 4)) - op.f[3], s.dr);
+    case SF_NODE_NORM_FENCE: return over_dr(len3(s.p) - op.f[0], fabsf(s.dr));
     case SF_NODE_BULB_FENCE: return bulb_fence(s.p, s.dr);
     default: return SF_INF;
     }
@@ -626,7 +703,9 @@ __device__ __forceinline__ float box_dist(float3 p, float3 half) {
 }
 // A hierarchy node's signed box distance (bvh.rs:19-24; WGSL _cluster_bound).
 __device__ __forceinline__ float cluster_bound(const float* nd, float3 p) {
-    return box_dist(p - mk3(__ldg(nd), __ldg(nd + 1), __ldg(nd + 2)), mk3(__ldg(nd + 3), __ldg(nd + 4), __ldg(nd + 5)));
+    // a row is 8 floats, 16-byte aligned: blocks and rows are multiples of 4 floats
+    const float4 a = __ldg(reinterpret_cast<const float4*>(nd)), b = __ldg(reinterpret_cast<const float4*>(nd) + 1);
+    return box_dist(p - mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y));
 }
 // The search over one Instances node's copies (graph_wgsl.rs:760-790): seeded at
 // the nearest leaf by a greedy descent, then a stackless preorder walk that skips
@@ -659,9 +738,8 @@ __device__ __forceinline__ bool inst_next(InstFrame& F) {
         const uint32_t j = uint32_t(leaf);
         // the copy's inverse affine rows: local point, per-axis scale and its minimum
         const float* r = F.rows + size_t(j) * 12u;
-        const float4 x = make_float4(__ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3));
-        const float4 y = make_float4(__ldg(r + 4), __ldg(r + 5), __ldg(r + 6), __ldg(r + 7));
-        const float4 z = make_float4(__ldg(r + 8), __ldg(r + 9), __ldg(r + 10), __ldg(r + 11));
+        const float4* rows = reinterpret_cast<const float4*>(r);
+        const float4 x = __ldg(rows), y = __ldg(rows + 1), z = __ldg(rows + 2);
         const float3 q = mk3(dot3(mk3(x.x, x.y, x.z), F.c) + x.w, dot3(mk3(y.x, y.y, y.z), F.c) + y.w,
                              dot3(mk3(z.x, z.y, z.z), F.c) + z.w);
         const float3 sc = mk3(rsqrtf(fmaf(x.z, x.z, fmaf(x.x, x.x, x.y * x.y))),
@@ -716,8 +794,30 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
     float3 loop_seed[SF_MAX_LOOP_DEPTH];
     float loop_seed_dr[SF_MAX_LOOP_DEPTH];
     int depth = 0;
-    DeRaw stack[SF_MAX_DIST_STACK];
+    // the distance stack: its top in registers, the sp - 1 entries below it in local memory
+    DeRaw below[SF_MAX_DIST_STACK - 1], top = raw_empty();
     int sp = 0;
+    auto push = [&](const DeRaw& r) {
+        if (sp > 0) below[sp - 1] = top;
+        top = r;
+        sp++;
+    };
+    // The nearest of the first operands that wait on the stack, k deep, for the Unions a
+    // branch is a second operand of (the lowering counts them). A Union keeps its first
+    // operand up to and including a tie, so a branch whose lower bound reaches this
+    // distance cannot be the sample, whatever its own value: its detail is left out, and
+    // a copy search starts from this distance instead of 1e30.
+    auto union_best = [&](uint32_t k) {
+        float u = SF_INF;
+        if (k > 0 && sp > 0) u = fminf(u, top.d);
+        for (uint32_t i = 1; i < k && int(i) < sp; ++i) u = fminf(u, below[sp - 1 - i].d);
+        return u;
+    };
+    // A lower bound that reaches it (never when no first operand waits, as in a leaf's own range).
+    auto out_of_reach = [&](float bound, uint32_t k) {
+        const float u = union_best(k);
+        return u < SF_INF && bound >= u;
+    };
     float3 seed_p = c;
     float seed_dr = 1.0f;
     const uint32_t lanes = __activemask();
@@ -729,6 +829,7 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
         if (at == 0xffffffffu) break;
         if (here != at) continue;
         const DeOp& op = P.ops[at];
+        bool search = false;  // an Instances node looks for its next copy
         switch (op.code) {
         case SF_OP_BEGIN:
             s.p = c; s.dr = 1.0f; s.iter = 0; s.t0 = s.t1 = s.t2 = s.t3 = SF_INF;
@@ -758,28 +859,26 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
             break;
         }
         case SF_OP_FENCE_OFF:
-            if (sp < SF_MAX_DIST_STACK) stack[sp++] = dist_from(s, SF_INF);
+            if (sp < SF_MAX_DIST_STACK) push(dist_from(s, SF_INF));
             break;
         case SF_OP_EMPTY:
-            if (sp < SF_MAX_DIST_STACK) stack[sp++] = raw_empty();
+            if (sp < SF_MAX_DIST_STACK) push(raw_empty());
             break;
         case SF_OP_TAG:
-            if (sp > 0) stack[sp - 1].material = op.a;
+            if (sp > 0) top.material = op.a;
             break;
         case SF_OP_BOUND:
-            if (sp > 0) stack[sp - 1].d = fmaxf(stack[sp - 1].d, box_fence(s.p, ld3(op.f), s.dr));
+            if (sp > 0) top.d = fmaxf(top.d, box_fence(s.p, ld3(op.f), s.dr));
             break;
         case SF_OP_BOUND_FAST: {
             if (sp >= SF_MAX_DIST_STACK) break;
             DeRaw b = raw_empty();
             b.d = box_fence(s.p, ld3(op.f), s.dr);
-            if (!exact && (probe || b.d > op.f[3])) {
+            if ((!exact && (probe || b.d > op.f[3])) || out_of_reach(b.d, op.a)) {
                 b.flags = 1;
-                stack[sp++] = b;
                 pc = op.b;  // past BOUND_END
-                break;
             }
-            stack[sp++] = b;
+            push(b);
             break;
         }
         case SF_OP_INST_BEGIN: {
@@ -796,11 +895,11 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
             if (F.skip) {
                 // empty space needs only the root fence (graph_wgsl.rs:769-771)
                 const float env = cluster_bound(F.bvh, c);
-                if (probe || env > F.margin) {
+                if (probe || env > F.margin || out_of_reach(env, uint32_t(op.f[5]))) {
                     DeRaw e = raw_empty();
                     e.d = env;
                     e.flags = 1;
-                    stack[sp++] = e;
+                    push(e);
                     pc = op.b;
                     fd--;
                     break;
@@ -818,39 +917,32 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
             F.seed_pass = true;
             F.chosen = op.a;
             F.best = raw_empty();
-            F.best.d = 1e30f;
-            if (inst_next(F)) { c = F.q; break; }  // the template follows with the copy's point
-            stack[sp++] = F.best;
-            pc = op.b;
-            fd--;
+            F.best.d = fminf(1e30f, union_best(uint32_t(op.f[5])));
+            search = true;
             break;
         }
         case SF_OP_INST_END: {
             if (sp < 1 || fd < 0) break;
             InstFrame& F = frames[fd];
-            DeRaw d = stack[--sp];
+            DeRaw d = top;
             d.d = fmaxf(d.d * F.w, F.fence);
             if (d.d < F.best.d || (d.d == F.best.d && F.j < F.chosen)) { F.best = d; F.chosen = F.j; }
-            if (inst_next(F)) { c = F.q; pc = op.a; break; }  // next copy: the template again
-            c = F.c;  // the point the search ran at (an outer copy's local point, nested)
-            stack[sp++] = F.best;
-            fd--;
+            if (--sp > 0) top = below[sp - 1];
+            search = true;
             break;
         }
         case SF_OP_BOUND_END:
             if (sp >= 2) {
-                DeRaw r = stack[sp - 1];
-                r.d = fmaxf(stack[sp - 2].d, r.d);
-                stack[sp - 2] = r;
+                top.d = fmaxf(below[sp - 2].d, top.d);
                 sp--;
             }
             break;
         case SF_OP_COMBINE:
-            if (sp >= 2) { stack[sp - 2] = combine_op(op.a, op.f[0], stack[sp - 2], stack[sp - 1]); sp--; }
+            if (sp >= 2) { top = combine_op(op.a, op.f[0], below[sp - 2], top); sp--; }
             break;
         default:
             if (op.code >= SF_NODE_SPHERE && op.code <= SF_NODE_BULB_FENCE) {
-                if (sp < SF_MAX_DIST_STACK) stack[sp++] = dist_from(s, fence_op(op, s));
+                if (sp < SF_MAX_DIST_STACK) push(dist_from(s, fence_op(op, s)));
             } else {
                 // outside any Iterate, AddSeed reinjects the point entering this node
                 if (depth == 0) { seed_p = s.p; seed_dr = s.dr; }
@@ -858,9 +950,22 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
             }
             break;
         }
+        if (search) {
+            InstFrame& F = frames[fd];
+            const bool begin = op.code == SF_OP_INST_BEGIN;
+            if (inst_next(F)) {  // the template runs at the copy's point
+                c = F.q;
+                pc = begin ? at : op.a;
+            } else {
+                c = F.c;  // the point the search ran at (an outer copy's local point, nested)
+                push(F.best);
+                pc = begin ? op.b : at;
+                fd--;
+            }
+        }
         ++pc;
     }
-    return sp > 0 ? stack[sp - 1] : raw_empty();
+    return sp > 0 ? top : raw_empty();
 }
 // The whole program: exact = false is the reference's de_sample (skippable Bounded
 // branches skipped outside their margin, the sample flagged); exact = true is

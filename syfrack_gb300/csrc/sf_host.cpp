@@ -375,6 +375,15 @@ struct Lowerer {
     // Instances node inside it skips either
     int template_depth = 0;
     bool template_exact = false;
+    // first operands of enabled Unions on the stack whose Union the branch being lowered
+    // reaches as (part of) the second operand through Unions and tags alone
+    uint32_t pending = 0;
+    struct Pending {  // sets pending for a subtree
+        uint32_t& p;
+        const uint32_t old;
+        Pending(Lowerer& l, uint32_t v) : p(l.pending), old(l.pending) { p = v; }
+        ~Pending() { p = old; }
+    };
 
     bool push(const DeOp& op) {
         if (P.n_ops >= SF_MAX_OPS) { err = "graph too large for the device program"; return false; }
@@ -465,9 +474,11 @@ struct Lowerer {
                 const uint32_t at = P.n_ops;
                 DeOp o = mk(SF_OP_BOUND_FAST);
                 std::memcpy(o.f, n.f, sizeof o.f);
+                o.a = pending;
                 if (!push(o)) return false;
                 stack_depth++;
                 max_stack = std::max(max_stack, stack_depth);
+                const Pending detail(*this, 0);
                 if (!dist(hb, b, guard + 1)) return false;
                 if (!push(mk(SF_OP_BOUND_END))) return false;
                 stack_depth--;
@@ -475,8 +486,9 @@ struct Lowerer {
                 P.fast_bounds++;
                 return true;
             }
+            if (!n.enabled) return dist(hb, b, guard + 1);
+            const Pending detail(*this, 0);
             if (!dist(hb, b, guard + 1)) return false;
-            if (!n.enabled) return true;
             if (!chain(ha, a)) return false;
             DeOp o = mk(SF_OP_BOUND);
             std::memcpy(o.f, n.f, sizeof o.f);
@@ -497,11 +509,13 @@ struct Lowerer {
             std::memcpy(o.f, n.f, 4 * sizeof(float));
             const bool skippable = !unsafe_bounds.count(src) && !template_exact;
             o.f[4] = skippable ? 1.f : 0.f;
+            o.f[5] = float(pending);
             pack_instances(g.placements.data() + n.u[0], n.u[1], n.f, *inst);
             if (!push(o)) return false;
             const bool outer_exact = template_exact;
             template_depth++;
             template_exact = !skippable;
+            const Pending copies(*this, 0);
             const bool ok = dist(ha, a, guard + 1);
             template_depth--;
             template_exact = outer_exact;
@@ -513,8 +527,14 @@ struct Lowerer {
             return true;
         }
         if (is_combine_kind(n.kind)) {
-            if (!dist(ha, a, guard + 1)) return false;
-            if (!n.enabled) return true;  // disabled: port 0 passes through (eval.rs:822)
+            if (!n.enabled) return dist(ha, a, guard + 1);  // disabled: port 0 passes through (eval.rs:822)
+            const bool is_union = n.kind == SF_NODE_UNION;
+            const uint32_t before = pending;
+            {
+                const Pending first(*this, is_union ? before : 0);
+                if (!dist(ha, a, guard + 1)) return false;
+            }
+            const Pending second(*this, is_union ? before + 1 : 0);
             if (!dist(hb, b, guard + 1)) return false;
             DeOp o = mk(SF_OP_COMBINE);
             o.a = n.kind;
@@ -539,7 +559,9 @@ struct Lowerer {
         if (n && n->enabled && n->kind == SF_NODE_UNION) {
             uint32_t a = 0, b = 0;
             const bool ha = g.input_of(src, 0, &a), hb = g.input_of(src, 1, &b);
-            if (!union_tree(ha, a, guard + 1) || !union_tree(hb, b, guard + 1)) return false;
+            if (!union_tree(ha, a, guard + 1)) return false;
+            const Pending second(*this, pending + 1);
+            if (!union_tree(hb, b, guard + 1)) return false;
             DeOp o = mk(SF_OP_COMBINE);
             o.a = n->kind;
             o.f[0] = n->f[0];
@@ -1389,6 +1411,7 @@ extern "C" sf_status sf_graph_compile(sf_context* c, const sf_graph_desc* d, sf_
     if (g->d_inst) e = cudaMemcpyAsync(g->d_inst, inst.data(), g->inst_bytes, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(g->d_prog, &g->prog, sizeof(DeProgram), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess && g->prog.n_ops) e = sf_launch_prepare_program(g->d_prog, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         ctx_free(c, g->d_prog, sizeof(DeProgram));
@@ -1420,6 +1443,7 @@ extern "C" sf_status sf_graph_update(sf_graph* g, const sf_graph_desc* d) {
     CU(cudaDeviceSynchronize());  // no launch on any stream (previews, server slots) may read what is replaced
     if (g->d_inst) CU(cudaMemcpyAsync(g->d_inst, inst.data(), g->inst_bytes, cudaMemcpyHostToDevice, g->ctx->stream));
     CU(cudaMemcpyAsync(g->d_prog, &P, sizeof P, cudaMemcpyHostToDevice, g->ctx->stream));
+    if (P.n_ops) CU(sf_launch_prepare_program(g->d_prog, g->ctx->stream));
     CU(cudaStreamSynchronize(g->ctx->stream));
     g->host = h;
     g->prog = P;

@@ -31,6 +31,11 @@ __global__ void __launch_bounds__(256) k_de_probe(const DeProgram* __restrict__ 
     }
 }
 
+// Once per upload of a program: the constants of its ops (prepare_op).
+__global__ void k_prepare_program(DeProgram* prog) {
+    for (uint32_t i = threadIdx.x; i < prog->n_ops; i += blockDim.x) prepare_op(prog->ops[i]);
+}
+
 // ------------------------------------------------------------------ persistent trace
 // Every lane holds one segment; a lane whose segment ends fetches the next work
 // item immediately (warp-aggregated), so all lanes keep evaluating the DE in
@@ -673,6 +678,10 @@ static unsigned grid_for(size_t n, unsigned threads, unsigned per_sm) {
     return want ? (unsigned)want : 1u;
 }
 
+cudaError_t sf_launch_prepare_program(DeProgram* prog, cudaStream_t st) {
+    k_prepare_program<<<1, 256, 0, st>>>(prog);
+    return cudaGetLastError();
+}
 cudaError_t sf_launch_de_probe(const DeProgram* prog, const float* x, const float* y, const float* z, size_t n,
                                float* dist, float* traps, uint32_t* iters, uint32_t* mats, cudaStream_t st) {
     if (!n) return cudaSuccess;

@@ -148,6 +148,8 @@ struct BatchTable {
 };
 
 // ---- launchers (return cudaError_t of the launch) ----
+// Follows every upload of a program with ops (a generic graph), on the same stream.
+cudaError_t sf_launch_prepare_program(DeProgram* prog, cudaStream_t st);
 cudaError_t sf_launch_de_probe(const DeProgram* prog, const float* x, const float* y, const float* z, size_t n,
                                float* dist, float* traps, uint32_t* iters, uint32_t* mats, cudaStream_t st);
 cudaError_t sf_launch_primary(const DeProgram* prog, const DevScene* scene, uint32_t width, uint32_t height,
