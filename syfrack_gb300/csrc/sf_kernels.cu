@@ -221,8 +221,9 @@ cudaError_t sf_launch_film_clear(FilmPlanes film, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ megakernel
-// The plain per-pixel integrator (pathtrace.wgsl:1203-1276): one thread per
-// pixel runs every sample's whole path with blocking marches.
+// The plain per-pixel integrator (pathtrace.wgsl:1203-1276): one thread per path, a
+// sample of a pixel, with blocking marches. A pixel's samples run in different blocks
+// (blockIdx.z): k_commit adds them in ascending order whichever ends first.
 static __device__ int march_full(const DeProgram& P, March& m, uint32_t max_steps, float safety, float accept,
                                  bool absolute, DeRaw& hit, unsigned long long& evals, unsigned long long& iters) {
     int r = march_check(m, max_steps, accept);
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(64) k_megakernel(const DeProgram* __restrict__
     unsigned long long evals = 0, iters = 0, segs = 0;
     const uint32_t stream = point_stream_of(S, px, py);
     const bool optics = (FEAT & SF_FEAT_RICH) && (S.rich & SF_RICH_OPTICS) != 0u;
-    for (uint32_t s = 0; s < g.samples; ++s) {
+    for (uint32_t s = blockIdx.z; s < g.samples; s += gridDim.z) {
         uint32_t sample = g.sample_start + s;
         PathState ps;
         path_begin(S, ps, px, py, sample);
@@ -728,7 +729,7 @@ cudaError_t sf_launch_commit(PathSoA soa, DispatchGeom g, FilmPlanes film, cudaS
 }
 cudaError_t sf_launch_megakernel(const DeProgram* prog, const DevScene* scene, uint32_t rich, PathSoA soa,
                                  DispatchGeom g, FilmPlanes film, unsigned long long* stats, cudaStream_t st) {
-    dim3 grid((g.tile_w + 7) / 8, (g.tile_h + 7) / 8);
+    dim3 grid((g.tile_w + 7) / 8, (g.tile_h + 7) / 8, g.samples < 65535u ? g.samples : 65535u);
     if (rich & SF_RICH_TEXTURE) k_megakernel<3><<<grid, 64, g.light_smem, st>>>(prog, scene, soa, g, film, stats);
     else if (rich) k_megakernel<1><<<grid, 64, g.light_smem, st>>>(prog, scene, soa, g, film, stats);
     else k_megakernel<0><<<grid, 64, g.light_smem, st>>>(prog, scene, soa, g, film, stats);
