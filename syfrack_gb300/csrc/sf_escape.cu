@@ -12,7 +12,8 @@
 // The traps (ring, stripe bands, final angle) are tolerance quantities (the
 // reference's own GPU parity bound is 0.006): for an integer stripe count k the
 // per-iteration sin(k atan2(y, x)) comes from the Chebyshev recurrence on
-// cos(theta), sin(theta) = z/|z|, and the ring distance uses |z| = |z|^2 rsqrt(|z|^2). With TRAPS = false only the
+// cos(theta), sin(theta) = z/|z| (the default 12 from the double angle, see z2_step), and
+// the ring distance uses |z| = |z|^2 rsqrt(|z|^2). With TRAPS = false only the
 // iteration count, smooth time and distance are produced.
 #include <cuda_runtime.h>
 
@@ -120,23 +121,21 @@ static __device__ __forceinline__ float sin_multiple(float c, float s, int k) {
     return sign * b;
 }
 
-// sin(12 theta), the default stripe count of PlanarFractal: the recurrence unrolled.
-static __device__ __forceinline__ float sin_12(float c, float s) {
-    const float c2 = 2.0f * c;
-    float a = 0.0f, b = s;
-#pragma unroll
-    for (int j = 1; j < 12; ++j) {
-        float t = fmaf(c2, b, -a);
-        a = b;
-        b = t;
-    }
-    return b;
+// sin(12 theta) / 4, the default stripe count of PlanarFractal, from the double angle:
+// with C = cos 2 theta and h = sin(2 theta) / 2, sin 3u = sin u (3 - 4 sin^2 u) and
+// cos 3u = cos u (1 - 4 sin^2 u) at u = 2 theta give
+// sin 12 theta = 4 (h C) ((3 - 16 h^2) (1 - 16 h^2)).
+// Against FP64 over 4 M angles: largest error 7.4e-6, rms 1.2e-6 (the 11-step
+// recurrence it replaces: 1.4e-5, 1.8e-6), in 7 operations after h and C instead of 12.
+static __device__ __forceinline__ float quarter_sin_12(float C, float h, float sum) {
+    const float q = h * h;
+    return fmaf(h * C, fmaf(-16.0f, q, 3.0f) * fmaf(-16.0f, q, 1.0f), sum);
 }
 
 // One iteration; true once the orbit has escaped or spent its iteration budget.
-// POW2: the power is 2 (z^2 as one complex square). SK12: the stripe count is 12.
+// POW2: the power is 2 (z^2 as one complex square).
 // o.stripe accumulates sin(k theta); the bands use 0.5 n + 0.5 * that sum.
-template <bool TRAPS, bool POW2, bool SK12 = false>
+template <bool TRAPS, bool POW2>
 static __device__ __forceinline__ bool esc_step(const EscParams& p, EscOrbit& o) {
     if (o.count >= p.iterations) return true;
     float r2 = FA(FM(o.zx, o.zx), FM(o.zy, o.zy));
@@ -150,8 +149,7 @@ static __device__ __forceinline__ bool esc_step(const EscParams& p, EscOrbit& o)
         o.ring = fminf(o.ring, fabsf(radius - p.trap_radius));
         float s = 0.0f;
         if (r2 > 0.0f) {
-            if (SK12) s = sin_12(o.zx * rinv, o.zy * rinv);
-            else if (p.stripe_k != SF_STRIPES_GENERAL) s = sin_multiple(o.zx * rinv, o.zy * rinv, p.stripe_k);
+            if (p.stripe_k != SF_STRIPES_GENERAL) s = sin_multiple(o.zx * rinv, o.zy * rinv, p.stripe_k);
             else s = sinf(p.stripes * atan2f(o.zy, o.zx));
         }
         o.stripe += s;
@@ -368,67 +366,171 @@ __global__ void __launch_bounds__(256) k_escape2d_root(const PlanarDev* __restri
 }
 
 // One tile of the canvas, escape families: each lane owns one pixel at a time and
-// takes the next pixel of the tile (warp-aggregated atomic on *work, which starts at
-// 0) as soon as its orbit ends, checking every ESC_CHUNK iterations, so lanes whose
-// pixels escape early do not idle beside interior pixels that run the whole budget.
+// takes another (warp-aggregated atomic on *work, which starts at 0) once its orbit has
+// ended, so lanes whose pixels escape early do not idle beside interior pixels that run
+// the whole budget. Orbits advance ESC_CHUNK iterations at a time. A finished lane waits
+// until ESC_REGEN lanes of its warp have finished, at most ESC_WAIT chunks, so that the
+// logarithms and angles of a pixel's end and the next pixel's set-up run for several
+// lanes at once.
 // Without TRAPS only dist, traps[0 .. n) (smooth time) and iters are written.
-constexpr int ESC_CHUNK = 16;
+constexpr int ESC_CHUNK = 16, ESC_REGEN = 8, ESC_WAIT = 4;
+enum { ESC_GENERAL = 0, ESC_POW2 = 1, ESC_Z2 = 2, ESC_SHIP = 3, ESC_PHOENIX = 4 };
 
-// Up to ESC_CHUNK iterations; true once the orbit has ended.
-template <bool TRAPS, bool POW2, bool SK12>
-static __device__ __forceinline__ bool esc_chunk(const EscParams& p, EscOrbit& o) {
+// One iteration of z^2 without twist at the default 12 stripes: Julia and Mandelbrot
+// (ESC_Z2), Burning Ship, Phoenix. r2 = |z|^2 of the point it leaves; the caller has
+// shown r2 to be a normal number at most bail_t. The arithmetic rounds as esc_step's,
+// bit for bit, with fewer instructions: the squares of |z|^2 serve the new real part
+// (|x|*|x| = x*x exactly), the imaginary part is fl(x*y) doubled (fl(x*y) + fl(y*x) =
+// 2 fl(x*y), fl(|x|*|y|) = |fl(x*y)|, and doubling is exact, so one fused multiply-add
+// rounds as the sum with c does), and the squares are a packed f32x2 multiply.
+// Instruction issue bounds it: about 21 issue slots an iteration with traps and 8
+// without, against 50 and 34 when every iteration tested for the end of the orbit and
+// the stripes ran the recurrence.
+struct Z2Orbit {
+    float x, y, qx, qy, ring, stripe4;
+};
+template <bool TRAPS, int MODE>
+static __device__ __forceinline__ void z2_step(const EscParams& p, float cx, float cy, Z2Orbit& o, float2 sq, float r2) {
+    const float m = FM(o.x, o.y), d = FS(sq.x, sq.y);
+    if (TRAPS) {
+        float rinv;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rinv) : "f"(r2));
+        o.ring = fminf(o.ring, fabsf(FM(r2, rinv) - p.trap_radius));
+        const float ir2 = rinv * rinv;
+        o.stripe4 = quarter_sin_12(d * ir2, m * ir2, o.stripe4);
+    }
+    float nx = FA(d, cx), ny = fmaf(2.0f, MODE == ESC_SHIP ? fabsf(m) : m, cy);
+    if (MODE == ESC_PHOENIX) {
+        nx = FA(nx, FM(o.qx, p.memory));
+        ny = FA(ny, FM(o.qy, p.memory));
+        o.qx = o.x;
+        o.qy = o.y;
+    }
+    o.x = nx;
+    o.y = ny;
+}
+
+// Up to ESC_CHUNK iterations of a z^2 orbit; true once it has ended. `checked` tests
+// every iteration; otherwise a whole chunk runs without a branch, only noting whether
+// some |z|^2 was past the bailout or not a normal number, and is done again from its
+// start, checked, if so: an orbit pays that once, at its end. The first chunk is
+// always checked (Mandelbrot and Burning Ship start at zero, and most orbits that
+// escape do so there).
+template <bool TRAPS, int MODE>
+static __device__ __forceinline__ bool esc_chunk_z2(const EscParams& p, EscOrbit& e) {
+    const float cx = e.cx, cy = e.cy, bt = p.bail_t;
+    const uint32_t left = p.iterations - e.count;  // count <= iterations
+    Z2Orbit o{e.zx, e.zy, e.qx, e.qy, e.ring, e.stripe};
+    bool ended = e.count == 0 || left < (uint32_t)ESC_CHUNK;  // or may end: run it checked
+    if (!ended) {
+#pragma unroll
+        for (int j = 0; j < ESC_CHUNK; ++j) {
+            const float2 sq = mul2(o.x, o.y, o.x, o.y);  // (x*x, y*y)
+            const float r2 = FA(sq.x, sq.y);
+            ended |= (TRAPS && !(r2 >= 1.17549435e-38f)) | (r2 > bt);
+            z2_step<TRAPS, MODE>(p, cx, cy, o, sq, r2);
+        }
+        if (!ended) {
+            e.count += ESC_CHUNK;
+        } else {
+            o = Z2Orbit{e.zx, e.zy, e.qx, e.qy, e.ring, e.stripe};
+        }
+    }
+    bool done = false;
+    if (ended) {
+        const int n = left < (uint32_t)ESC_CHUNK ? (int)left : ESC_CHUNK;
+        int j = 0;
+        for (; j < n; ++j) {
+            const float2 sq = mul2(o.x, o.y, o.x, o.y);
+            const float r2 = FA(sq.x, sq.y);
+            if (r2 > bt) {
+                e.escaped = true;
+                break;
+            }
+            if (TRAPS && !(r2 >= 1.17549435e-38f)) {
+                // zero, subnormal or not a number: the directions as esc_step takes them
+                const float rinv = rsqrtf(r2);
+                o.ring = fminf(o.ring, fabsf((r2 > 0.0f ? r2 * rinv : 0.0f) - p.trap_radius));
+                if (r2 > 0.0f) {
+                    const float ux = o.x * rinv, uy = o.y * rinv;
+                    o.stripe4 = quarter_sin_12(fmaf(ux, ux, -(uy * uy)), ux * uy, o.stripe4);
+                }
+                z2_step<false, MODE>(p, cx, cy, o, sq, r2);
+            } else {
+                z2_step<TRAPS, MODE>(p, cx, cy, o, sq, r2);
+            }
+        }
+        e.count += (uint32_t)j;
+        done = e.escaped || e.count >= p.iterations;
+    }
+    e.zx = o.x;
+    e.zy = o.y;
+    e.qx = o.qx;
+    e.qy = o.qy;
+    e.ring = o.ring;
+    e.stripe = o.stripe4;
+    return done;
+}
+
+template <bool TRAPS, int MODE>
+static __device__ __forceinline__ bool esc_advance(const EscParams& p, EscOrbit& o) {
+    if (MODE >= ESC_Z2) return esc_chunk_z2<TRAPS, MODE>(p, o);
     for (int j = 0; j < ESC_CHUNK; ++j)
-        if (esc_step<TRAPS, POW2, SK12>(p, o)) return true;
+        if (esc_step<TRAPS, MODE == ESC_POW2>(p, o)) return true;
     return false;
 }
 
-// The common tile: z^2 without twist (Julia, Mandelbrot or, SHIP, Burning Ship), the
-// default 12 stripes. The budget is checked once per chunk instead of per iteration.
-// The orbit's arithmetic rounds as esc_step's, bit for bit, with fewer instructions:
-// the squares x*x, y*y of |z|^2 serve the new real part (|x|*|x| = x*x exactly), the
-// imaginary part is fl(x*y) doubled (fl(x*y) + fl(y*x) = 2 fl(x*y), and
-// fl(|x|*|y|) = |fl(x*y)|), and the paired products and the sum with c are packed
-// f32x2 operations, each lane rounded as a binary32 multiply or add.
-template <bool TRAPS, bool SHIP>
-static __device__ __forceinline__ bool esc_chunk_z2(const EscParams& p, EscOrbit& o) {
-    const uint32_t left = p.iterations - o.count;  // count <= iterations
-    const int n = left < (uint32_t)ESC_CHUNK ? (int)left : ESC_CHUNK;
-    float zx = o.zx, zy = o.zy, ring = o.ring, stripe = o.stripe;
-    const float cx = o.cx, cy = o.cy, bt = p.bail_t, tr = p.trap_radius;
-    int j = 0;
-    bool escaped = false;
-    for (; j < n; ++j) {
-        const float2 sq = mul2(zx, zy, zx, zy);  // (x*x, y*y)
-        const float r2 = FA(sq.x, sq.y);
-        if (r2 > bt) {
-            escaped = true;
-            break;
-        }
-        if (TRAPS) {
-            const float rinv = rsqrtf(r2);
-            ring = fminf(ring, fabsf((r2 > 0.0f ? r2 * rinv : 0.0f) - tr));
-            if (r2 > 0.0f) {
-                const float2 u = mul2(zx, zy, rinv, rinv);  // z / |z|
-                stripe += sin_12(u.x, u.y);
+// The pixels of a tile, one persistent loop per mode (the modes' code apart keeps each
+// loop's registers and instructions its own).
+template <bool TRAPS, int MODE>
+static __device__ __forceinline__ unsigned long long esc_pixels(const PlanarDev& F, const CanvasDev& K, const EscParams& p,
+                                                                uint32_t tile_x, uint32_t tile_y, uint32_t tile_w,
+                                                                uint32_t n, uint32_t sample, float* dist, float* traps,
+                                                                uint32_t* iters, uint32_t* work) {
+    unsigned long long total_iters = 0;
+    const float scale = __fdiv_rn(6.0f, K.zoom);
+    EscOrbit o;
+    uint32_t pix = 0;
+    enum { IDLE, BUSY, DONE, OUT };
+    uint32_t state = IDLE;
+    int waited = 0;
+    for (;;) {
+        // every lane of the warp reaches this point together
+        const uint32_t ready = __ballot_sync(FULL_MASK, state == IDLE || state == DONE);
+        const uint32_t busy = __ballot_sync(FULL_MASK, state == BUSY);
+        if (ready == 0u && busy == 0u) break;
+        if (ready != 0u && (__popc(ready) >= ESC_REGEN || ++waited >= ESC_WAIT || busy == 0u)) {
+            waited = 0;
+            if (state == DONE) {
+                float tr[4], d;
+                const float stripe = MODE >= ESC_Z2 ? 4.0f * o.stripe : o.stripe;
+                planar_finish<TRAPS>(F, o.zx, o.zy, o.escaped, false, o.count, o.count, float(F.iterations), o.ring,
+                                     0.5f * float(o.count) + 0.5f * stripe, d, tr);
+                store_pixel(dist, traps, iters, n, pix, d, tr, o.count, TRAPS);
+                total_iters += o.count;
+                state = IDLE;
+            }
+            const uint32_t got = warp_fetch(work, state == IDLE);
+            if (state == IDLE) {
+                if (got < n) {
+                    pix = got;
+                    float px, py, qx, qy;
+                    canvas_point(K, scale, tile_x + pix % tile_w, tile_y + pix / tile_w, sample, qx, qy);
+                    planar_map(F, qx, qy, px, py);
+                    esc_init(F, px, py, o);
+                    state = BUSY;
+                } else {
+                    state = OUT;
+                }
             }
         }
-        const float m = FM(zx, zy);
-        const float mm = SHIP ? fabsf(m) : m;
-        const float2 z = add2(FS(sq.x, sq.y), FA(mm, mm), cx, cy);
-        zx = z.x;
-        zy = z.y;
+        if (state == BUSY && esc_advance<TRAPS, MODE>(p, o)) state = DONE;
     }
-    o.zx = zx;
-    o.zy = zy;
-    o.ring = ring;
-    o.stripe = stripe;
-    o.count += (uint32_t)j;
-    o.escaped = escaped;
-    return escaped || o.count >= p.iterations;
+    return total_iters;
 }
 
 template <bool TRAPS>
-__global__ void __launch_bounds__(256, 5) k_escape2d(const PlanarDev* __restrict__ fg,
+__global__ void __launch_bounds__(256, 4) k_escape2d(const PlanarDev* __restrict__ fg,
                                                      const CanvasDev* __restrict__ cg, uint32_t tile_x,
                                                      uint32_t tile_y, uint32_t tile_w, uint32_t tile_h,
                                                      uint32_t sample, float* dist, float* traps, uint32_t* iters,
@@ -439,49 +541,19 @@ __global__ void __launch_bounds__(256, 5) k_escape2d(const PlanarDev* __restrict
     stage_pod(K, cg);
     __syncthreads();
     const uint32_t n = tile_w * tile_h;
-    unsigned long long total_iters = 0;
-    const float scale = __fdiv_rn(6.0f, K.zoom);
     const EscParams p = esc_params(F);
-    const bool pow2 = p.power == 2, sk12 = p.stripe_k == 12;
-    const bool z2 = pow2 && sk12 && !p.rotate && !p.phoenix;
-    EscOrbit o;
-    uint32_t pix = 0;
-    bool busy = false, live = true;
-    for (;;) {
-        // every lane of the warp reaches this point together
-        bool want = live && !busy;
-        uint32_t got = warp_fetch(work, want);
-        if (want) {
-            if (got < n) {
-                pix = got;
-                float px, py, qx, qy;
-                canvas_point(K, scale, tile_x + pix % tile_w, tile_y + pix / tile_w, sample, qx, qy);
-                planar_map(F, qx, qy, px, py);
-                esc_init(F, px, py, o);
-                busy = true;
-            } else {
-                live = false;
-            }
-        }
-        if (!__any_sync(FULL_MASK, busy)) break;
-        if (busy) {
-            bool done;
-            if (z2 && p.ship) done = esc_chunk_z2<TRAPS, true>(p, o);
-            else if (z2) done = esc_chunk_z2<TRAPS, false>(p, o);
-            else if (pow2 && sk12) done = esc_chunk<TRAPS, true, true>(p, o);
-            else if (pow2) done = esc_chunk<TRAPS, true, false>(p, o);
-            else done = esc_chunk<TRAPS, false, false>(p, o);
-            if (done) {
-                float tr[4], d;
-                planar_finish<TRAPS>(F, o.zx, o.zy, o.escaped, false, o.count, o.count, float(F.iterations), o.ring,
-                                     0.5f * float(o.count) + 0.5f * o.stripe, d, tr);
-                store_pixel(dist, traps, iters, n, pix, d, tr, o.count, TRAPS);
-                total_iters += o.count;
-                busy = false;
-            }
-        }
-    }
-    warp_stat(&stats[SF_STAT_DE_ITERS], total_iters);
+    // the z^2 loop: 12 stripes, no twist, and a bailout whose |z|^2 stays finite, so that
+    // an orbit has passed it before any product overflows
+    const bool z2 = p.power == 2 && p.stripe_k == 12 && !p.rotate && p.bail_t <= 1e37f;
+    unsigned long long total;
+#define ESC_RUN(MODE) esc_pixels<TRAPS, MODE>(F, K, p, tile_x, tile_y, tile_w, n, sample, dist, traps, iters, work)
+    if (z2 && p.ship) total = ESC_RUN(ESC_SHIP);
+    else if (z2 && p.phoenix) total = ESC_RUN(ESC_PHOENIX);
+    else if (z2) total = ESC_RUN(ESC_Z2);
+    else if (p.power == 2) total = ESC_RUN(ESC_POW2);
+    else total = ESC_RUN(ESC_GENERAL);
+#undef ESC_RUN
+    warp_stat(&stats[SF_STAT_DE_ITERS], total);
 }
 
 static unsigned escape_grid(size_t n, unsigned per_sm) {
@@ -511,10 +583,10 @@ cudaError_t sf_launch_escape2d(const PlanarDev* f, const CanvasDev* canvas, uint
         k_escape2d_root<false><<<escape_grid(n, 8), 256, 0, st>>>(f, canvas, tile_x, tile_y, tile_w, tile_h, sample,
                                                                    dist, traps, iters, stats);
     else if (with_traps)
-        k_escape2d<true><<<escape_grid(n, 5), 256, 0, st>>>(f, canvas, tile_x, tile_y, tile_w, tile_h, sample, dist,
+        k_escape2d<true><<<escape_grid(n, 4), 256, 0, st>>>(f, canvas, tile_x, tile_y, tile_w, tile_h, sample, dist,
                                                              traps, iters, stats, work);
     else
-        k_escape2d<false><<<escape_grid(n, 5), 256, 0, st>>>(f, canvas, tile_x, tile_y, tile_w, tile_h, sample, dist,
+        k_escape2d<false><<<escape_grid(n, 4), 256, 0, st>>>(f, canvas, tile_x, tile_y, tile_w, tile_h, sample, dist,
                                                               traps, iters, stats, work);
     return cudaGetLastError();
 }
