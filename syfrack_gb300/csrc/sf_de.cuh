@@ -268,7 +268,10 @@ __device__ __forceinline__ DeRaw raw_empty() {
 
 // ------------------------------------------------------------------ specialised forms
 // Mandelbulb: Iterate{Trap, Power, AddOrigin} -> BulbFence (graphs/mandelbulb.ron).
-__device__ __forceinline__ DeRaw de_bulb(const FormParams& f, float3 p) {
+// NORM_MIN0: the bundled trap (slot 0, Norm, Minimum). N: the power, 8, or 0 to read it
+// from the parameters; with both fixed the iteration has no choices left to make.
+template <bool NORM_MIN0, uint32_t N>
+__device__ __forceinline__ DeRaw de_bulb_t(const FormParams& f, float3 p) {
     DeRaw s = raw_empty();
     const float3 c = p;
     float dr = 1.0f;
@@ -278,9 +281,13 @@ __device__ __forceinline__ DeRaw de_bulb(const FormParams& f, float3 p) {
         // any error by n
         float r = len3(p);
         if (r > f.bailout) break;
-        float v = f.trap_measure == SF_MEASURE_NORM ? r : trap_measure(f.trap_measure, p);
-        trap_update(s, f.trap_slot, f.trap_mode, v);
-        power_op(p, dr, r, f.power, f.power_int);
+        if (NORM_MIN0) {
+            s.t0 = fminf(s.t0, r);
+        } else {
+            float v = f.trap_measure == SF_MEASURE_NORM ? r : trap_measure(f.trap_measure, p);
+            trap_update(s, f.trap_slot, f.trap_mode, v);
+        }
+        power_op(p, dr, r, f.power, N ? N : f.power_int);
         p = p + c;
         dr += 1.0f;
         s.iter++;
@@ -288,6 +295,11 @@ __device__ __forceinline__ DeRaw de_bulb(const FormParams& f, float3 p) {
     s.d = bulb_fence(p, dr);
     s.material = f.material;
     return s;
+}
+__device__ __forceinline__ DeRaw de_bulb(const FormParams& f, float3 p) {
+    if (f.trap_measure == SF_MEASURE_NORM && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM)
+        return f.power_int == 8u ? de_bulb_t<true, 8u>(f, p) : de_bulb_t<true, 0u>(f, p);
+    return de_bulb_t<false, 0u>(f, p);
 }
 
 
@@ -376,15 +388,19 @@ __device__ __forceinline__ DeRaw de_box(const FormParams& f, float3 p) {
 }
 
 // Menger: Iterate{MengerFold, Trap} -> Box (graphs/menger.ron).
-__device__ __forceinline__ DeRaw de_menger(const FormParams& f, float3 p) {
+// NORM_MIN0: the bundled trap (slot 0, Norm, Minimum) kept as min |p|^2; the |p|^2 it
+// takes after the fold is the next iteration's bailout test, formed once.
+template <bool NORM_MIN0>
+__device__ __forceinline__ DeRaw de_menger_t(const FormParams& f, float3 p) {
     DeRaw s = raw_empty();
     float dr = 1.0f;
     const uint32_t n = f.iterations;
     const float sc = f.scale;
     const float3 off = mk3(f.offset[0], f.offset[1], f.offset[2]);
     const bool sq = f.trap_squared != 0;
+    float pp = NORM_MIN0 ? dot3(p, p) : 0.0f, t0 = SF_INF;
     for (uint32_t i = 0; i < n; ++i) {
-        if (dot3(p, p) > f.bailout_t) break;
+        if ((NORM_MIN0 ? pp : dot3(p, p)) > f.bailout_t) break;
         float3 z = abs3(p);
         if (z.x < z.y) z = mk3(z.y, z.x, z.z);
         if (z.x < z.z) z = mk3(z.z, z.y, z.x);
@@ -393,14 +409,24 @@ __device__ __forceinline__ DeRaw de_menger(const FormParams& f, float3 p) {
         if (z.z < -0.5f * off.z * (sc - 1.0f)) z.z += off.z * (sc - 1.0f);
         p = z;
         dr *= sc;
-        float v = sq ? dot3(p, p) : trap_measure(f.trap_measure, p);
-        trap_update(s, f.trap_slot, f.trap_mode, v);
+        if (NORM_MIN0) {
+            pp = dot3(p, p);
+            t0 = fminf(t0, pp);
+        } else {
+            float v = sq ? dot3(p, p) : trap_measure(f.trap_measure, p);
+            trap_update(s, f.trap_slot, f.trap_mode, v);
+        }
         s.iter++;
     }
     s.d = box_fence(p, mk3(f.fence[0], f.fence[1], f.fence[2]), dr);
     s.material = f.material;
-    if (sq) trap_sqrt(s, f.trap_slot);
+    if (NORM_MIN0) s.t0 = sqrtf(t0);
+    else if (sq) trap_sqrt(s, f.trap_slot);
     return s;
+}
+__device__ __forceinline__ DeRaw de_menger(const FormParams& f, float3 p) {
+    if (f.trap_squared && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM) return de_menger_t<true>(f, p);
+    return de_menger_t<false>(f, p);
 }
 
 // ------------------------------------------------------------------ generic interpreter

@@ -1561,8 +1561,9 @@ extern "C" sf_status sf_primary_trace(sf_graph* g, const sf_primary_desc* d, flo
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_work, 0, 4, c->stream);
     if (e == cudaSuccess) {
         LaunchTimer t(c, true);
-        e = sf_launch_primary(g->d_prog, dS, d->width, d->height, d->max_steps, d->rule, d->eps, d->t_far,
-                              d->normal_mode, dt, ds, dn, c->d_work, c->d_stats, 1, c->stream);
+        const PrimaryLaunch pl{d->width, d->height, d->max_steps, d->rule, d->normal_mode, d->eps, d->t_far,
+                               dt, ds, dn, c->d_work, c->d_stats};
+        e = sf_launch_primary(g->prog.form, g->d_prog, dS, pl, c->stream);
     }
     // t, steps and normals are contiguous after the scene: one copy into the staging
     if (e == cudaSuccess) e = ensure_stage(c, n * 20);

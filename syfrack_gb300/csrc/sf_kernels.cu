@@ -36,129 +36,6 @@ __global__ void k_prepare_program(DeProgram* prog) {
     for (uint32_t i = threadIdx.x; i < prog->n_ops; i += blockDim.x) prepare_op(prog->ops[i]);
 }
 
-// ------------------------------------------------------------------ persistent trace
-// Every lane holds one segment; a lane whose segment ends fetches the next work
-// item immediately (warp-aggregated), so all lanes keep evaluating the DE in
-// lockstep instead of waiting for the warp's longest march. Surface hits of
-// continuation rays run the four normal taps through the same DE call.
-enum { LANE_IDLE = 0, LANE_CONT = 1, LANE_SHADOW = 2, LANE_NORMAL = 3, LANE_DONE = 4 };
-
-// ------------------------------------------------------------------ primary rays
-// Primary rays through pixel centres (control.wgsl:270-273), the same relaxed
-// march with a fixed-epsilon (rule 1) or cone-relative (rule 0) hit test, then a
-// 6-tap central (normal_mode 0) or 4-tap tetrahedral (1) normal.
-__device__ __forceinline__ float3 central_offset(uint32_t i) {
-    float sgn = (i & 1u) ? -1.0f : 1.0f;
-    uint32_t a = i >> 1;
-    return mk3(a == 0 ? sgn : 0.f, a == 1 ? sgn : 0.f, a == 2 ? sgn : 0.f);
-}
-
-__global__ void __launch_bounds__(256) k_primary(const DeProgram* __restrict__ prog_g,
-                                                 const DevScene* __restrict__ scene_g, uint32_t width, uint32_t height,
-                                                 uint32_t max_steps, int rule, float eps, float t_far, int normal_mode,
-                                                 float* t_out, uint32_t* steps_out, float* n_out,
-                                                 uint32_t* work_counter, unsigned long long* stats, int persistent) {
-    __shared__ DeProgram P;
-    __shared__ DevScene S;
-    stage_program(P, prog_g);
-    stage_pod(S, scene_g);
-    __syncthreads();
-    const uint32_t total = width * height;
-    const float cone = S.tan_half * 2.0f / float(width);
-    const float accept = rule == 1 ? eps : cone * S.pixel_tolerance;
-    const bool absolute = rule == 1;
-    const uint32_t taps = normal_mode == 0 ? 6u : 4u;
-    const float3 fw = ld3(S.forward), rt = ld3(S.right), up = ld3(S.up), org = ld3(S.origin);
-    uint32_t state = LANE_IDLE, pix = 0, tap = 0;
-    March m;
-    float3 hp = mk3(0.f, 0.f, 0.f), grad = mk3(0.f, 0.f, 0.f);
-    float hstep = 0.f, thit = 0.f;
-    unsigned long long n_eval = 0, n_iter = 0, n_steps = 0;
-    uint32_t next_static = blockIdx.x * blockDim.x + threadIdx.x;
-    while (true) {
-        uint32_t w;
-        if (persistent) {
-            w = warp_fetch(work_counter, state == LANE_IDLE);
-        } else {
-            w = next_static;
-        }
-        if (state == LANE_IDLE) {
-            if (!persistent) next_static += gridDim.x * blockDim.x;
-            if (w >= total) {
-                state = LANE_DONE;
-            } else {
-                pix = w;
-                uint32_t px = pix % width, py = pix / width;
-                float ndcx = ((float(px) + 0.5f) / float(width)) * 2.0f - 1.0f;
-                float ndcy = ((float(py) + 0.5f) / float(height)) * 2.0f - 1.0f;
-                float3 rd = normalize3(fw + rt * (ndcx * S.tan_half) + up * (-ndcy * S.tan_half / S.aspect));
-                march_begin(m, org, rd, t_far);
-                state = LANE_CONT;
-            }
-        }
-        if (__all_sync(FULL_MASK, state == LANE_DONE)) break;
-        if (state == LANE_CONT || state == LANE_NORMAL) {
-            int r = MARCH_CONTINUE;
-            if (state == LANE_CONT) r = march_check(m, max_steps, accept);
-            DeRaw s;
-            bool evaluated = false;
-            if (r == MARCH_CONTINUE) {
-                float3 qp = state == LANE_NORMAL
-                                ? hp + (normal_mode == 0 ? central_offset(tap) : tetra_offset(tap)) * hstep
-                                : m.ro + m.rd * m.t;
-                s = de_raw(P, qp);
-                evaluated = true;
-                n_eval++;
-                n_iter += s.iter;
-                if (state == LANE_CONT && needs_exact(s, m.t, S.step_scale, accept, absolute)) {
-                    s = de_raw_exact(P, qp);
-                    n_eval++;
-                    n_iter += s.iter;
-                }
-            }
-            if (state == LANE_NORMAL) {
-                grad = grad + (normal_mode == 0 ? central_offset(tap) : tetra_offset(tap)) * s.d;
-                if (++tap == taps) {
-                    float3 n = normalize3(grad);
-                    t_out[pix] = thit;
-                    n_out[pix] = n.x;
-                    n_out[total + pix] = n.y;
-                    n_out[2 * total + pix] = n.z;
-                    state = LANE_IDLE;
-                }
-            } else {
-                bool at_budget = !evaluated;
-                if (evaluated) {
-                    r = march_update(m, s.d, s.flags, S.step_scale, accept, absolute);
-                    if (r == MARCH_CONTINUE) r = march_check(m, max_steps, accept), at_budget = r != MARCH_CONTINUE;
-                    if (r == MARCH_HIT && !at_budget) m.cand_t = m.t;
-                }
-                if (r != MARCH_CONTINUE) {
-                    steps_out[pix] = m.i;
-                    n_steps += m.i;
-                    if (r == MARCH_HIT) {
-                        thit = m.cand_t;
-                        hp = m.ro + m.rd * thit;
-                        hstep = fmaxf(thit * cone * 0.5f, 1e-4f) * S.pixel_tolerance;
-                        grad = mk3(0.f, 0.f, 0.f);
-                        tap = 0;
-                        state = LANE_NORMAL;
-                    } else {
-                        t_out[pix] = -1.0f;
-                        n_out[pix] = 0.f;
-                        n_out[total + pix] = 0.f;
-                        n_out[2 * total + pix] = 0.f;
-                        state = LANE_IDLE;
-                    }
-                }
-            }
-        }
-    }
-    warp_stat(&stats[SF_STAT_DE_EVALS], n_eval);
-    warp_stat(&stats[SF_STAT_DE_ITERS], n_iter);
-    warp_stat(&stats[SF_STAT_STEPS], n_steps);
-}
-
 // ------------------------------------------------------------------ wavefront stages
 __global__ void __launch_bounds__(256) k_generate(const DevScene* __restrict__ scene_g, PathSoA soa, DispatchGeom g,
                                                   uint32_t* counts) {
@@ -689,15 +566,14 @@ cudaError_t sf_launch_de_probe(const DeProgram* prog, const float* x, const floa
     k_de_probe<<<grid_for(n, 256, 8), 256, 0, st>>>(prog, x, y, z, n, dist, traps, iters, mats);
     return cudaGetLastError();
 }
-cudaError_t sf_launch_primary(const DeProgram* prog, const DevScene* scene, uint32_t width, uint32_t height,
-                              uint32_t max_steps, int rule, float eps, float t_far, int normal_mode, float* t_out,
-                              uint32_t* steps_out, float* normal_out, uint32_t* work_counter,
-                              unsigned long long* stats, int persistent, cudaStream_t st) {
-    size_t n = (size_t)width * height;
-    unsigned blocks = persistent ? (unsigned)sf_device_sm_count() * 8u : (unsigned)((n + 255) / 256);
-    k_primary<<<blocks, 256, 0, st>>>(prog, scene, width, height, max_steps, rule, eps, t_far, normal_mode, t_out,
-                                      steps_out, normal_out, work_counter, stats, persistent);
-    return cudaGetLastError();
+cudaError_t sf_launch_primary(uint32_t form, const DeProgram* prog, const DevScene* scene, const PrimaryLaunch& pl,
+                              cudaStream_t st) {
+    switch (form) {
+    case SF_FORM_BULB: return sf_launch_primary_bulb(prog, scene, pl, st);
+    case SF_FORM_BOX: return sf_launch_primary_box(prog, scene, pl, st);
+    case SF_FORM_MENGER: return sf_launch_primary_menger(prog, scene, pl, st);
+    default: return sf_launch_primary_any(prog, scene, pl, st);
+    }
 }
 cudaError_t sf_launch_generate(const DevScene* scene, PathSoA soa, DispatchGeom g, uint32_t* counts, cudaStream_t st) {
     k_generate<<<(g.paths + 255) / 256, 256, g.light_smem, st>>>(scene, soa, g, counts);

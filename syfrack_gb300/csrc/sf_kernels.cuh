@@ -85,6 +85,19 @@ struct TraceLaunch {
     uint32_t optics;              // 1: the scene has dielectric materials (the optics trace kernel)
 };
 
+// One frame of primary rays: planes of width * height values (n: three planes).
+// *work is the pixel counter of the launch and must be 0 when it starts.
+struct PrimaryLaunch {
+    uint32_t width, height, max_steps;
+    int rule, normal_mode;  // rule 1: fixed epsilon; normal_mode 0: central, 1: tetrahedral
+    float eps, t_far;
+    float* t;
+    uint32_t* steps;
+    float* n;
+    uint32_t* work;
+    unsigned long long* stats;
+};
+
 struct FilmPlanes {
     float4* accum;  // sum of (L, 1) per sample
     float* depth;   // first-hit distance, -1 for a miss (sample 0)
@@ -152,10 +165,13 @@ struct BatchTable {
 cudaError_t sf_launch_prepare_program(DeProgram* prog, cudaStream_t st);
 cudaError_t sf_launch_de_probe(const DeProgram* prog, const float* x, const float* y, const float* z, size_t n,
                                float* dist, float* traps, uint32_t* iters, uint32_t* mats, cudaStream_t st);
-cudaError_t sf_launch_primary(const DeProgram* prog, const DevScene* scene, uint32_t width, uint32_t height,
-                              uint32_t max_steps, int rule, float eps, float t_far, int normal_mode, float* t_out,
-                              uint32_t* steps_out, float* normal_out, uint32_t* work_counter,
-                              unsigned long long* stats, int persistent, cudaStream_t st);
+// Primary rays, one instantiation per form (sf_trace_<form>.cu).
+cudaError_t sf_launch_primary(uint32_t form, const DeProgram* prog, const DevScene* scene, const PrimaryLaunch& pl,
+                              cudaStream_t st);
+cudaError_t sf_launch_primary_bulb(const DeProgram*, const DevScene*, const PrimaryLaunch&, cudaStream_t);
+cudaError_t sf_launch_primary_box(const DeProgram*, const DevScene*, const PrimaryLaunch&, cudaStream_t);
+cudaError_t sf_launch_primary_menger(const DeProgram*, const DevScene*, const PrimaryLaunch&, cudaStream_t);
+cudaError_t sf_launch_primary_any(const DeProgram*, const DevScene*, const PrimaryLaunch&, cudaStream_t);
 cudaError_t sf_launch_generate(const DevScene* scene, PathSoA soa, DispatchGeom g, uint32_t* counts, cudaStream_t st);
 // Persistent trace kernel, one instantiation per form (sf_trace_<form>.cu).
 cudaError_t sf_launch_trace(uint32_t form, const DeProgram* prog, const DevScene* scene, PathSoA soa, TraceLaunch tl,
