@@ -230,8 +230,8 @@ cudaError_t sf_launch_ref_orbit(double cx, double cy, uint32_t max_iter, double 
 // entries), then its parallel split into the hi/lo arrays.
 cudaError_t sf_launch_ref_orbit_split(double cx, double cy, uint32_t max_iter, double bailout, double2* z,
                                       float2* orbit_lo, float2* orbit_f, uint32_t* orbit_len, cudaStream_t st);
-// *work is the pixel counter of the launch and must be 0 when it starts. c_lo: the
-// centre's part below the orbit's c_ref, added to every pixel's offset.
+// *work is the pixel counter of the launch and must be 0 when it starts; orbit_f is
+// 32-byte aligned. c_lo: the centre's part below the orbit's c_ref, added to every pixel's offset.
 cudaError_t sf_launch_perturb(const float2* orbit_lo, const float2* orbit_f, const uint32_t* orbit_len, uint32_t width,
                               uint32_t height, float pitch, float2 c_lo, uint32_t max_iter, float bailout,
                               uint32_t* iters, float* smooth, unsigned long long* stats, uint32_t* work,

@@ -31,6 +31,8 @@ struct NoAllocScratch {
     unsigned long long stats[SF_STAT_COUNT];
 };
 
+static_assert(offsetof(NoAllocScratch, orbit_f) % 32 == 0, "the perturbation kernel reads the orbit in 32-byte loads");
+
 // 1 MB per device. In host code this name is only a stand-in for the symbol:
 // kernels receive the address cudaGetSymbolAddress returns for the current device.
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;

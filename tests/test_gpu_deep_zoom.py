@@ -106,3 +106,18 @@ def test_centre_lo_moves_the_view_below_an_fp64_ulp(gpu_ctx, oracle_mod):
     print(f"centre lo: view changed on {(a != b).mean():.3f} of pixels; match vs binary128 lo=0 "
           f"{(a[idx] == ta).mean():.3f}, with lo {(b[idx] == tb).mean():.3f}")
     assert (b[idx] == tb).mean() >= 0.6
+
+
+@pytest.mark.parametrize("max_iter", [1, 2, 7, 8, 9, 12, 16, 17, 40])
+def test_budgets_around_the_chunk(gpu_ctx, max_iter):
+    """Budgets around the 8 iterations a pixel runs without a branch and the 4 orbit
+    entries of a load. At this width a count differs from FP64 direct iteration only
+    where binary32's rounding, grown by the orbit, decides the last step: under a
+    hundredth of the pixels. The host's orbit gives the device's frame bit for bit."""
+    args = dict(center_hi=(-0.75, 0.1), center_lo=(0.0, 0.0), width_units=2.5, width=101, height=67,
+                max_iter=max_iter)
+    a = deep_zoom(gpu_ctx, **args, reference_f64=True)
+    b = deep_zoom(gpu_ctx, **args, orbit="host")
+    assert (a["iterations"] == a["iterations_f64"]).mean() >= 0.99
+    for k in ("iterations", "smooth", "rebases"):
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)

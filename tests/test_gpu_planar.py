@@ -124,3 +124,23 @@ def test_escape2d_without_traps_keeps_counts(gpu_ctx):
     assert lean.traps is None and lean.distance is None
     np.testing.assert_array_equal(lean.iterations, full["iterations"])
     np.testing.assert_array_equal(lean.smooth, full["traps"][0])
+
+
+@pytest.mark.parametrize("iterations", [1, 15, 16, 17, 32, 49])
+@pytest.mark.parametrize("family", ["Julia", "Mandelbrot", "BurningShip", "Phoenix"])
+def test_escape2d_around_the_chunk(gpu_ctx, oracle_mod, family, iterations):
+    """Budgets around the 16 iterations an orbit runs without a branch: counts bit for
+    bit, traps within the 0.006 of the reference's own parity test on all but one pixel
+    in a thousand (a ring or band next to a discontinuity)."""
+    c = Canvas(width=97, height=61, center=(-0.4, -0.1), zoom=1.7)
+    f = PlanarFractal(family=family, iterations=iterations)
+    out = escape2d(gpu_ctx, f, c)
+    ref = oracle_mod.planar(oracle_params(oracle_mod, f), canvas_points(c), precision=32)
+    np.testing.assert_array_equal(out["iterations"].ravel(), ref["iterations"])
+    d = np.abs(out["traps"].reshape(4, -1).T - ref["traps"])
+    assert np.quantile(d, 0.999) <= 0.006
+    # the general loop (five stripes) runs the same orbit
+    g = escape2d(gpu_ctx, PlanarFractal(family=family, iterations=iterations, stripes=5.0), c)
+    np.testing.assert_array_equal(g["iterations"], out["iterations"])
+    np.testing.assert_array_equal(g["distance"], out["distance"])
+    np.testing.assert_array_equal(g["traps"][0], out["traps"][0])
