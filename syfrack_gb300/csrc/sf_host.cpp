@@ -660,7 +660,6 @@ void detect_form(const HostGraph& g, DeProgram& P) {
         f.fold_k_min = f.fixed_radius2 / f.min_radius2;
         f.fold_clamped = f.fold_k_min >= 1.0f ? 1u : 0u;
         f.scale = body[3]->f[0];
-        f.abs_scale = std::fabs(f.scale);
         f.fence[0] = fence->f[0];
         P.form = SF_FORM_BOX;
     } else if (fence->kind == SF_NODE_BOX && kinds({SF_NODE_MENGER_FOLD, SF_NODE_TRAP})) {
@@ -1811,6 +1810,7 @@ extern "C" sf_status sf_session_dispatch(sf_session* s, sf_tile tile, uint32_t s
             tl.regen = s->regen;
             tl.lane_stats = c->lane_stats ? 1u : 0u;
             tl.optics = (rich & SF_RICH_OPTICS) ? 1u : 0u;
+            tl.fp = s->graph->prog.fp;
             LaunchTimer t(c, true);
             CU(sf_launch_trace(s->graph->prog.form, s->graph->d_prog, s->d_scene, s->soa, tl, c->d_stats, blocks,
                                int(s->min_blocks), s->light_smem, st));

@@ -19,6 +19,14 @@ enum { TL_IDLE = 0, TL_MARCH = 1, TL_CAND = 2, TL_NORMAL = 3, TL_DONE = 4, TL_IN
 #define SF_FORM_ANY 99u
 #define SF_FORM_MIXED 98u  // any of the three iterated forms, chosen per lane
 
+// fp: the form's constants, P's own or those of the launch (TraceLaunch.fp).
+template <int FORM>
+__device__ __forceinline__ DeRaw de_form(const DeProgram& P, const FormParams& fp, float3 p) {
+    if constexpr (FORM == SF_FORM_BULB) return de_bulb(fp, p);
+    else if constexpr (FORM == SF_FORM_BOX) return de_box(fp, p);
+    else if constexpr (FORM == SF_FORM_MENGER) return de_menger(fp, p);
+    else return de_raw(P, p);
+}
 template <int FORM>
 __device__ __forceinline__ DeRaw de_form(const DeProgram& P, float3 p) {
     if constexpr (FORM == SF_FORM_BULB) return de_bulb(P.fp, p);
@@ -193,7 +201,8 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* 
                         item = it & 0x7fffffffu;
                         shadow = (it >> 31) != 0;
                     }
-                    path = shadow ? item % cap : item;
+                    path = item;
+                    while (path >= cap) path -= cap;  // of shadow row k * cap + path
                     if constexpr (MULTI) {
                         const BatchJob& job = bt.jobs[find_job(begins, bt.n_jobs, path)];
                         Pl = job.prog;
@@ -234,7 +243,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* 
                 s = exact_state ? de_raw_exact(*Pl, q) : de_form<FORM>(*Pl, q);
             else if constexpr (MULTI) s = de_form<FORM>(*Pl, q);
             else if constexpr (FORM == SF_FORM_ANY && OPTICS) s = exact_state ? de_raw_exact(P, q) : de_form<FORM>(P, q);
-            else s = de_form<FORM>(P, q);
+            else s = de_form<FORM>(P, tl.fp, q);
             n_eval++;
             n_iter += s.iter;
             if constexpr (FORM == SF_FORM_ANY) {
