@@ -382,6 +382,9 @@ typedef struct sf_primary_desc {
 } sf_primary_desc;
 sf_status sf_primary_trace(sf_graph* graph, const sf_primary_desc* desc, float* t_out, uint32_t* steps_out,
                            float* normal_out);
+/* Same, with the normals as (pixel, 3) rows in normal_out. */
+sf_status sf_primary_trace_rows(sf_graph* graph, const sf_primary_desc* desc, float* t_out, uint32_t* steps_out,
+                                float* normal_out);
 
 /* ------------------------------------------------------------------ statistics & timing */
 typedef struct sf_stats {

@@ -127,6 +127,7 @@ SIGNATURES = {
     "sf_de_probe": [vp, fp, C.c_size_t, P(abi.sf_de_sample)],
     "sf_de_probe_device": [vp, vp, vp, vp, C.c_size_t, vp, vp, vp, vp],
     "sf_primary_trace": [vp, P(sf_primary_desc), fp, up, fp],
+    "sf_primary_trace_rows": [vp, P(sf_primary_desc), fp, up, fp],
     "sf_session_create": [vp, vp, P(abi.sf_scene_desc), P(abi.sf_render_config), P(vp)],
     "sf_session_dispatch": [vp, abi.sf_tile, u32],
     "sf_session_step": [vp, u32, P(C.c_int)],

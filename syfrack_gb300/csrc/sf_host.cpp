@@ -24,6 +24,7 @@
 #include <vector>
 
 #include <sys/stat.h>
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include "../../include/syfrack_gpu.h"
@@ -799,17 +800,52 @@ sf_status wait_stream(cudaStream_t st, uint32_t timeout_ms) {
         if (e != cudaErrorNotReady) return cuda_fail(e, "stream");
         double el = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         if (timeout_ms && el > timeout_ms) return fail(SF_ERR_TIMEOUT, "dispatch exceeded its time limit");
-        std::this_thread::sleep_for(std::chrono::microseconds(200));
+        // a small frame takes a millisecond or two: poll without sleeping meanwhile
+        if (el < 2.0) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(200));
     }
 }
 
-// Runs f(begin, end) over [0, n) on up to 8 host threads (one below 1 M items).
-template <class F> void host_parallel(size_t n, F&& f) {
-    const size_t parts = std::min<size_t>(8, std::max<size_t>(1, n >> 20));
-    if (parts == 1) { f(size_t(0), n); return; }
+// Runs f(begin, end) over [0, n) on up to `most` host threads, one for each `grain` items.
+template <class F> void host_parallel(size_t n, size_t grain, F&& f, size_t most = 8) {
+    const size_t parts = std::min<size_t>(most, std::max<size_t>(1, n / grain));
     std::vector<std::thread> pool;
-    for (size_t k = 0; k < parts; ++k) pool.emplace_back([&, k] { f(n * k / parts, n * (k + 1) / parts); });
+    size_t k = 1;
+    try {
+        for (; k < parts; ++k) pool.emplace_back([&, k] { f(n * k / parts, n * (k + 1) / parts); });
+    } catch (...) {  // no thread to be had: the rest runs here
+    }
+    f(size_t(0), n / parts);
+    if (k < parts) f(n * k / parts, n);
     for (auto& t : pool) t.join();
+}
+
+// Results go from the device straight into the caller's (pageable) buffers: this
+// platform's copy engine reads and writes host memory through its page tables at link
+// speed (100 MB in 0.56 ms, as into pinned memory), and a second pass over the data by
+// host threads cost 5 to 9 ms. What is slow is memory that has never been touched, whose
+// pages the copy then maps one by one (3.8 ms for 100 MB): populate_pages maps them, after
+// the launch and while the device works, without changing what they hold (1.4 ms on 3
+// threads; touching each page with a read and a write took 33 ms, the read mapping the
+// zero page that the write then replaces). Where the kernel does not know the request it
+// is without effect.
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+struct HostOut {
+    void* p;
+    size_t bytes;
+};
+void populate_pages(std::initializer_list<HostOut> outs) {
+    static const size_t page = size_t(std::max<long>(sysconf(_SC_PAGESIZE), 4096));
+    for (const HostOut& o : outs) {
+        if (!o.p || !o.bytes) continue;
+        const uintptr_t b = reinterpret_cast<uintptr_t>(o.p) / page;
+        const size_t pages = (reinterpret_cast<uintptr_t>(o.p) + o.bytes + page - 1) / page - b;
+        host_parallel(pages, std::max<size_t>((size_t(16) << 20) / page, 1), [&](size_t k, size_t end) {
+            madvise(reinterpret_cast<void*>((b + k) * page), (end - k) * page, MADV_POPULATE_WRITE);
+        }, 4);
+    }
 }
 
 // The context's pinned staging at `bytes` or more (stage_mu held).
@@ -1479,7 +1515,7 @@ extern "C" sf_status sf_de_probe_device(sf_graph* g, const float* x, const float
     sf_context* c = g->ctx;
     cudaSetDevice(c->device);
     LaunchTimer t(c, true);
-    CU(sf_launch_de_probe(g->d_prog, x, y, z, n, dist, traps, iters, mats, c->stream));
+    CU(sf_launch_de_probe(g->d_prog, ProbeArrays{x, y, z, dist, traps, iters, mats, 1, 1, n}, n, c->stream));
     return SF_OK;
 }
 
@@ -1489,47 +1525,32 @@ extern "C" sf_status sf_de_probe(sf_graph* g, const float* xyz, size_t n, sf_de_
     if (!xyz || !out) return fail(SF_ERR_INVALID, "null buffer");
     sf_context* c = g->ctx;
     cudaSetDevice(c->device);
-    std::vector<float> soa(3 * n);
-    for (size_t i = 0; i < n; ++i) {
-        soa[i] = xyz[3 * i];
-        soa[n + i] = xyz[3 * i + 1];
-        soa[2 * n + i] = xyz[3 * i + 2];
-    }
-    size_t bytes = n * (3 + 1 + 4) * sizeof(float) + 2 * n * sizeof(uint32_t);
-    void* buf = nullptr;
-    sf_status s = ctx_alloc(c, bytes, &buf);
-    if (s != SF_OK) return s;
-    float* d_in = static_cast<float*>(buf);
-    float* d_dist = d_in + 3 * n;
-    float* d_traps = d_dist + n;
-    uint32_t* d_iter = reinterpret_cast<uint32_t*>(d_traps + 4 * n);
-    uint32_t* d_mat = d_iter + n;
-    std::vector<float> h_dist(n), h_traps(4 * n);
-    std::vector<uint32_t> h_iter(n), h_mat(n);
-    cudaError_t e = cudaMemcpyAsync(d_in, soa.data(), 3 * n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+    static_assert(sizeof(sf_de_sample) == 28, "distance, traps, iterations and material, packed");
+    // points and samples as the caller holds them, in the context's scratch
+    std::lock_guard<std::mutex> lk(c->stage_mu);
+    const size_t in_bytes = (n * 12 + 255) & ~size_t(255);
+    if (const sf_status s = ensure_scratch(c, in_bytes + n * sizeof(sf_de_sample)); s != SF_OK) return s;
+    float* d_in = static_cast<float*>(c->scratch);
+    float* d_out = reinterpret_cast<float*>(static_cast<char*>(c->scratch) + in_bytes);
+    cudaError_t e = cudaMemcpyAsync(d_in, xyz, n * 12, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
         LaunchTimer t(c, true);
-        e = sf_launch_de_probe(g->d_prog, d_in, d_in + n, d_in + 2 * n, n, d_dist, d_traps, d_iter, d_mat, c->stream);
+        uint32_t* u = reinterpret_cast<uint32_t*>(d_out);
+        const ProbeArrays io{d_in, d_in + 1, d_in + 2, d_out, d_out + 1, u + 5, u + 6, 3, 7, 1};
+        e = sf_launch_de_probe(g->d_prog, io, n, c->stream);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_dist.data(), d_dist, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_traps.data(), d_traps, 4 * n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_iter.data(), d_iter, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_mat.data(), d_mat, n * 4, cudaMemcpyDeviceToHost, c->stream);
+    populate_pages({{out, n * sizeof(sf_de_sample)}});
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(out, d_out, n * sizeof(sf_de_sample), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    ctx_free(c, buf, bytes);
     if (e != cudaSuccess) return cuda_fail(e, "sf_de_probe");
-    for (size_t i = 0; i < n; ++i) {
-        out[i].distance = h_dist[i];
-        for (int k = 0; k < 4; ++k) out[i].traps[k] = h_traps[k * n + i];
-        out[i].iterations = h_iter[i];
-        out[i].material = h_mat[i];
-    }
     return SF_OK;
 }
 
 // ------------------------------------------------------------------ ABI: primary rays
-extern "C" sf_status sf_primary_trace(sf_graph* g, const sf_primary_desc* d, float* t_out, uint32_t* steps_out,
-                                      float* normal_out) {
+// rows: normals as (pixel, 3) rows instead of three planes.
+static sf_status primary_trace(sf_graph* g, const sf_primary_desc* d, float* t_out, uint32_t* steps_out,
+                               float* normal_out, bool rows) {
     if (!g || !d) return fail(SF_ERR_INVALID, "null argument");
     if (!d->width || !d->height) return fail(SF_ERR_INVALID, "empty image");
     if (!t_out || !steps_out || !normal_out) return fail(SF_ERR_INVALID, "null output");
@@ -1548,7 +1569,7 @@ extern "C" sf_status sf_primary_trace(sf_graph* g, const sf_primary_desc* d, flo
     DevScene S;
     scene_dev(sd, rc, g->info, S);
     const size_t bytes = sizeof(DevScene) + n * (1 + 1 + 3) * 4;
-    // the context's scratch and pinned staging, kept between calls
+    // the context's scratch, kept between calls
     std::lock_guard<std::mutex> lk(c->stage_mu);
     if (const sf_status s = ensure_scratch(c, bytes); s != SF_OK) return s;
     void* buf = c->scratch;
@@ -1561,21 +1582,24 @@ extern "C" sf_status sf_primary_trace(sf_graph* g, const sf_primary_desc* d, flo
     if (e == cudaSuccess) {
         LaunchTimer t(c, true);
         const PrimaryLaunch pl{d->width, d->height, d->max_steps, d->rule, d->normal_mode, d->eps, d->t_far,
-                               dt, ds, dn, c->d_work, c->d_stats};
+                               dt, ds, dn, rows ? size_t(3) : size_t(1), rows ? size_t(1) : n, c->d_work, c->d_stats};
         e = sf_launch_primary(g->prog.form, g->d_prog, dS, pl, c->stream);
     }
-    // t, steps and normals are contiguous after the scene: one copy into the staging
-    if (e == cudaSuccess) e = ensure_stage(c, n * 20);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->stage, dt, n * 20, cudaMemcpyDeviceToHost, c->stream);
+    populate_pages({{t_out, n * 4}, {steps_out, n * 4}, {normal_out, n * 12}});
+    if (e == cudaSuccess) e = cudaMemcpyAsync(t_out, dt, n * 4, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(steps_out, ds, n * 4, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(normal_out, dn, n * 12, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "sf_primary_trace");
-    const char* st = static_cast<const char*>(c->stage);
-    host_parallel(n, [&](size_t b, size_t end) {
-        std::memcpy(t_out + b, st + b * 4, (end - b) * 4);
-        std::memcpy(steps_out + b, st + n * 4 + b * 4, (end - b) * 4);
-        std::memcpy(normal_out + 3 * b, st + n * 8 + b * 12, (end - b) * 12);
-    });
     return SF_OK;
+}
+extern "C" sf_status sf_primary_trace(sf_graph* g, const sf_primary_desc* d, float* t_out, uint32_t* steps_out,
+                                      float* normal_out) {
+    return primary_trace(g, d, t_out, steps_out, normal_out, false);
+}
+extern "C" sf_status sf_primary_trace_rows(sf_graph* g, const sf_primary_desc* d, float* t_out, uint32_t* steps_out,
+                                           float* normal_out) {
+    return primary_trace(g, d, t_out, steps_out, normal_out, true);
 }
 
 // ------------------------------------------------------------------ sessions
@@ -1908,57 +1932,44 @@ extern "C" sf_status sf_session_tiles(sf_session* s, sf_tile* tiles, uint32_t ca
 }
 
 namespace sfh {
-// Film readback through the context's pinned staging: the device planes arrive at
-// full link speed, then the host threads copy them into the caller's (pageable)
-// buffers and derive color = accum.rgb / max(count, 1) with alpha 1
-// (RenderOutput.color). A film without the volume layer split (no fog) has a zero
-// volume contribution: volume and moments are (0, 0, 0, samples) and surface = accum.
+// Film readback into the caller's buffers. color = accum.rgb / max(count, 1) with alpha 1
+// (RenderOutput.color); a film without the volume layer split (no fog) has a zero volume
+// contribution: volume and moments are (0, 0, 0, samples) and surface = accum. These
+// planes receive accum and are derived in place by the host threads.
 cudaError_t film_readback(sf_context* c, const FilmPlanes& f, const sf_film_planes& out, cudaStream_t st) {
+    (void)c;
     const size_t px = size_t(f.width) * f.height;
     const bool split = f.vol != nullptr;
-    const bool need_acc = out.accum || out.color || (!split && (out.volume || out.moments || out.surface));
-    const bool need_vol = split && (out.volume || out.moments || out.surface);
-    const size_t bytes = (need_acc ? px * 16 : 0) + (out.depth ? px * 4 : 0) + (out.aux ? px * 16 : 0) +
-                         (need_vol ? px * 48 : 0);
-    if (!bytes) return cudaSuccess;
-    std::lock_guard<std::mutex> lk(c->stage_mu);
-    if (cudaError_t e = ensure_stage(c, bytes); e != cudaSuccess) return e;
-    float* acc = static_cast<float*>(c->stage);
-    float* depth = acc + (need_acc ? px * 4 : 0);
-    float* aux = depth + (out.depth ? px : 0);
-    float* vol = aux + (out.aux ? px * 4 : 0);  // volume | moments | surface (contiguous on the device)
+    populate_pages({{out.accum, px * 16}, {out.depth, px * 4}, {out.aux, px * 16}, {out.volume, px * 16},
+                 {out.moments, px * 16}, {out.surface, px * 16}, {out.color, px * 16}});
     cudaError_t e = cudaSuccess;
-    if (need_acc) e = cudaMemcpyAsync(acc, f.accum, px * 16, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && out.depth) e = cudaMemcpyAsync(depth, f.depth, px * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && out.aux) e = cudaMemcpyAsync(aux, f.aux, px * 16, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && need_vol) e = cudaMemcpyAsync(vol, f.vol, px * 48, cudaMemcpyDeviceToHost, st);
+    auto copy = [&](float* to, const void* from, size_t bytes) {
+        if (to && e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, st);
+    };
+    copy(out.accum, f.accum, px * 16);
+    copy(out.depth, f.depth, px * 4);
+    copy(out.aux, f.aux, px * 16);
+    copy(out.color, f.accum, px * 16);
+    copy(out.volume, split ? f.vol : f.accum, px * 16);
+    copy(out.moments, split ? f.vmom : f.accum, px * 16);
+    copy(out.surface, split ? f.surf : f.accum, px * 16);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
-    host_parallel(px, [&](size_t b, size_t end) {
-        const size_t n = end - b;
-        if (out.accum) std::memcpy(out.accum + 4 * b, acc + 4 * b, n * 16);
-        if (out.depth) std::memcpy(out.depth + b, depth + b, n * 4);
-        if (out.aux) std::memcpy(out.aux + 4 * b, aux + 4 * b, n * 16);
-        if (split) {
-            if (out.volume) std::memcpy(out.volume + 4 * b, vol + 4 * b, n * 16);
-            if (out.moments) std::memcpy(out.moments + 4 * b, vol + 4 * (px + b), n * 16);
-            if (out.surface) std::memcpy(out.surface + 4 * b, vol + 4 * (2 * px + b), n * 16);
-        } else if (out.surface) {
-            std::memcpy(out.surface + 4 * b, acc + 4 * b, n * 16);
-        }
-        for (size_t i = b; i < end; ++i) {
-            const float cnt = acc[4 * i + 3];
-            if (out.color) {
-                const float d = std::max(cnt, 1.0f);
-                out.color[4 * i] = acc[4 * i] / d;
-                out.color[4 * i + 1] = acc[4 * i + 1] / d;
-                out.color[4 * i + 2] = acc[4 * i + 2] / d;
-                out.color[4 * i + 3] = 1.0f;
+    float* const zero[2] = {split ? nullptr : out.volume, split ? nullptr : out.moments};
+    if (!out.color && !zero[0] && !zero[1]) return cudaSuccess;
+    host_parallel(px, size_t(1) << 16, [&](size_t b, size_t end) {
+        if (out.color)
+            for (size_t i = b; i < end; ++i) {
+                float* const q = out.color + 4 * i;
+                const float d = std::max(q[3], 1.0f);
+                q[0] = q[0] / d;
+                q[1] = q[1] / d;
+                q[2] = q[2] / d;
+                q[3] = 1.0f;
             }
-            if (split) continue;
-            if (out.volume) { out.volume[4 * i] = out.volume[4 * i + 1] = out.volume[4 * i + 2] = 0.0f; out.volume[4 * i + 3] = cnt; }
-            if (out.moments) { out.moments[4 * i] = out.moments[4 * i + 1] = out.moments[4 * i + 2] = 0.0f; out.moments[4 * i + 3] = cnt; }
-        }
+        for (float* z : zero)
+            if (z)
+                for (size_t i = b; i < end; ++i) z[4 * i] = z[4 * i + 1] = z[4 * i + 2] = 0.0f;
     });
     return cudaSuccess;
 }
@@ -2274,7 +2285,7 @@ extern "C" sf_status sf_escape2d(sf_context* c, const sf_planar_desc* f, const s
     K.height = canvas->height;
     K.seed = uint32_t(canvas->seed) ^ uint32_t(canvas->seed >> 32);
     size_t bytes = 768 + n * 4 * 6;  // descriptors | pixel counter | outputs
-    // the context's device scratch and pinned staging, kept between calls
+    // the context's device scratch, kept between calls
     std::unique_lock<std::mutex> lk(c->stage_mu);
     st = ensure_scratch(c, bytes);
     if (st != SF_OK) return st;
@@ -2293,19 +2304,12 @@ extern "C" sf_status sf_escape2d(sf_context* c, const sf_planar_desc* f, const s
         e = sf_launch_escape2d(dF, dK, tile.x, tile.y, tile.w, tile.h, sample, dd, dt, di, c->d_stats, dW, 1,
                                F.family == 3 || F.family == 4, c->stream);
     }
-    // distance, traps and iterations are contiguous: one copy into the pinned staging,
-    // then host threads split it into the caller's arrays
-    if (e == cudaSuccess) e = ensure_stage(c, n * 24);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->stage, dd, n * 24, cudaMemcpyDeviceToHost, c->stream);
+    populate_pages({{dist, n * 4}, {traps, n * 16}, {iters, n * 4}});
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dist, dd, n * 4, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(traps, dt, n * 16, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(iters, di, n * 4, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "sf_escape2d");
-    const char* stg = static_cast<const char*>(c->stage);
-    host_parallel(n, [&](size_t b0, size_t b1) {
-        std::memcpy(dist + b0, stg + b0 * 4, (b1 - b0) * 4);
-        for (int k = 0; k < 4; ++k)  // traps are four planes of n
-            std::memcpy(traps + k * n + b0, stg + (n + k * n + b0) * 4, (b1 - b0) * 4);
-        std::memcpy(iters + b0, stg + (5 * n + b0) * 4, (b1 - b0) * 4);
-    });
     return SF_OK;
 }
 
@@ -2361,9 +2365,15 @@ extern "C" sf_status sf_deep_zoom(sf_context* c, const sf_deep_zoom_desc* d, uin
     const size_t Zb = d->orbit_mode == SF_ORBIT_DEVICE ? ((M * 16 + 255) & ~size_t(255)) : 0;
     const size_t z_off = (2 * Mb + 256 + n * 8 * (reference_f64 ? 2 : 1) + 255) & ~size_t(255);
     size_t bytes = z_off + Zb;
+    // the context's scratch, kept between calls, for frames up to 8K; larger ones allocate
+    const bool kept = bytes <= (size_t(512) << 20);
+    std::unique_lock<std::mutex> lk(c->stage_mu, std::defer_lock);
+    if (kept) lk.lock();
     void* buf = nullptr;
-    sf_status st = ctx_alloc(c, bytes, &buf);
+    sf_status st = kept ? ensure_scratch(c, bytes) : ctx_alloc(c, bytes, &buf);
     if (st != SF_OK) return st;
+    if (kept) buf = c->scratch;
+    else lk.lock();
     char* b = static_cast<char*>(buf);
     float2* olo = reinterpret_cast<float2*>(b);
     float2* of = reinterpret_cast<float2*>(b + Mb);
@@ -2382,9 +2392,7 @@ extern "C" sf_status sf_deep_zoom(sf_context* c, const sf_deep_zoom_desc* d, uin
     unsigned long long before[SF_STAT_COUNT];
     e = cudaMemcpyAsync(before, c->d_stats, sizeof before, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, 4, c->stream);
-    const size_t planes = reference_f64 ? 4 : 2;
-    std::unique_lock<std::mutex> lk(c->stage_mu);
-    if (e == cudaSuccess) e = ensure_stage(c, std::max(2 * Mb + 16, n * 4 * planes));
+    if (e == cudaSuccess && d->orbit_mode != SF_ORBIT_DEVICE) e = ensure_stage(c, 2 * Mb + 16);
     if (e == cudaSuccess && d->orbit_mode == SF_ORBIT_DEVICE) {
         LaunchTimer t(c, false);
         e = sf_launch_ref_orbit_split(cx, cy, d->max_iter, d->bailout, oz, olo, of, olen, c->stream);
@@ -2419,23 +2427,17 @@ extern "C" sf_status sf_deep_zoom(sf_context* c, const sf_deep_zoom_desc* d, uin
         e = sf_launch_direct_f64(cx, cy, d->center_lo[0], d->center_lo[1], d->width, d->height, pitch, d->max_iter,
                                  d->bailout, di64, ds64, c->stream);
     }
-    // the output planes are contiguous from di: one copy into the pinned staging (after
-    // the orbit's upload from it, in stream order), then host threads split it into the
-    // caller's arrays
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->stage, di, n * 4 * planes, cudaMemcpyDeviceToHost, c->stream);
+    const size_t n64 = reference_f64 ? n * 4 : 0;
+    populate_pages({{iters, n * 4}, {smooth, n * 4}, {iters64, n64}, {smooth64, n64}});
+    if (e == cudaSuccess) e = cudaMemcpyAsync(iters, di, n * 4, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(smooth, ds, n * 4, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && n64) e = cudaMemcpyAsync(iters64, di64, n64, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && n64) e = cudaMemcpyAsync(smooth64, ds64, n64, cudaMemcpyDeviceToHost, c->stream);
     unsigned long long after[SF_STAT_COUNT];
     if (e == cudaSuccess) e = cudaMemcpyAsync(after, c->d_stats, sizeof after, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    ctx_free(c, buf, bytes);
+    if (!kept) ctx_free(c, buf, bytes);
     if (e != cudaSuccess) return cuda_fail(e, "sf_deep_zoom");
-    {
-        const char* stg = static_cast<const char*>(c->stage);
-        void* outs[4] = {iters, smooth, iters64, smooth64};
-        host_parallel(n, [&](size_t b0, size_t b1) {
-            for (size_t k = 0; k < planes; ++k)
-                std::memcpy(static_cast<char*>(outs[k]) + b0 * 4, stg + k * n * 4 + b0 * 4, (b1 - b0) * 4);
-        });
-    }
     lk.unlock();
     if (rebases) *rebases = after[SF_STAT_STEPS] - before[SF_STAT_STEPS];
     return SF_OK;

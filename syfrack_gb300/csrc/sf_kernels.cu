@@ -13,21 +13,20 @@ static unsigned grid_for(size_t n, unsigned threads, unsigned per_sm);
 
 // ------------------------------------------------------------------ DE probe
 // de_probe.wgsl:9-17 / Renderer::probe_distances: one thread per point.
-__global__ void __launch_bounds__(256) k_de_probe(const DeProgram* __restrict__ prog_g, const float* __restrict__ x,
-                                                  const float* __restrict__ y, const float* __restrict__ z, size_t n,
-                                                  float* dist, float* traps, uint32_t* iters, uint32_t* mats) {
+__global__ void __launch_bounds__(256) k_de_probe(const DeProgram* __restrict__ prog_g, ProbeArrays io, size_t n) {
     __shared__ DeProgram P;
     stage_program(P, prog_g);
     __syncthreads();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        DeSampleF s = de_finalize(P, de_raw_exact_search(P, mk3(x[i], y[i], z[i])));
-        dist[i] = s.d;
-        traps[i] = s.traps[0];
-        traps[n + i] = s.traps[1];
-        traps[2 * n + i] = s.traps[2];
-        traps[3 * n + i] = s.traps[3];
-        iters[i] = s.iter;
-        mats[i] = s.material;
+        const size_t a = i * io.in, o = i * io.out;
+        DeSampleF s = de_finalize(P, de_raw_exact_search(P, mk3(io.x[a], io.y[a], io.z[a])));
+        io.dist[o] = s.d;
+        io.traps[o] = s.traps[0];
+        io.traps[o + io.trap] = s.traps[1];
+        io.traps[o + 2 * io.trap] = s.traps[2];
+        io.traps[o + 3 * io.trap] = s.traps[3];
+        io.iters[o] = s.iter;
+        io.mats[o] = s.material;
     }
 }
 
@@ -612,10 +611,9 @@ cudaError_t sf_launch_prepare_program(DeProgram* prog, cudaStream_t st) {
     k_prepare_program<<<1, 256, 0, st>>>(prog);
     return cudaGetLastError();
 }
-cudaError_t sf_launch_de_probe(const DeProgram* prog, const float* x, const float* y, const float* z, size_t n,
-                               float* dist, float* traps, uint32_t* iters, uint32_t* mats, cudaStream_t st) {
+cudaError_t sf_launch_de_probe(const DeProgram* prog, const ProbeArrays& io, size_t n, cudaStream_t st) {
     if (!n) return cudaSuccess;
-    k_de_probe<<<grid_for(n, 256, 8), 256, 0, st>>>(prog, x, y, z, n, dist, traps, iters, mats);
+    k_de_probe<<<grid_for(n, 256, 8), 256, 0, st>>>(prog, io, n);
     return cudaGetLastError();
 }
 cudaError_t sf_launch_primary(uint32_t form, const DeProgram* prog, const DevScene* scene, const PrimaryLaunch& pl,

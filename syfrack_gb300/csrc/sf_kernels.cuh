@@ -89,8 +89,8 @@ struct TraceLaunch {
     FormParams fp;
 };
 
-// One frame of primary rays: planes of width * height values (n: three planes).
-// *work is the pixel counter of the launch and must be 0 when it starts.
+// One frame of primary rays: planes of width * height values; component k of a pixel's
+// normal is at n[pixel * n_pixel + k * n_part]. *work is the pixel counter of the launch and must be 0 when it starts.
 struct PrimaryLaunch {
     uint32_t width, height, max_steps;
     int rule, normal_mode;  // rule 1: fixed epsilon; normal_mode 0: central, 1: tetrahedral
@@ -98,6 +98,7 @@ struct PrimaryLaunch {
     float* t;
     uint32_t* steps;
     float* n;
+    size_t n_pixel, n_part;
     uint32_t* work;
     unsigned long long* stats;
 };
@@ -167,8 +168,15 @@ struct BatchTable {
 // ---- launchers (return cudaError_t of the launch) ----
 // Follows every upload of a program with ops (a generic graph), on the same stream.
 cudaError_t sf_launch_prepare_program(DeProgram* prog, cudaStream_t st);
-cudaError_t sf_launch_de_probe(const DeProgram* prog, const float* x, const float* y, const float* z, size_t n,
-                               float* dist, float* traps, uint32_t* iters, uint32_t* mats, cudaStream_t st);
+// Points and samples of a probe: value i of an array is at i * in (x, y, z) or i * out,
+// trap k at i * out + k * trap (planes: 1, 1, n; interleaved sf_de_sample rows: 3, 7, 1).
+struct ProbeArrays {
+    const float *x, *y, *z;
+    float *dist, *traps;
+    uint32_t *iters, *mats;
+    size_t in, out, trap;
+};
+cudaError_t sf_launch_de_probe(const DeProgram* prog, const ProbeArrays& io, size_t n, cudaStream_t st);
 // Primary rays, one instantiation per form (sf_trace_<form>.cu).
 cudaError_t sf_launch_primary(uint32_t form, const DeProgram* prog, const DevScene* scene, const PrimaryLaunch& pl,
                               cudaStream_t st);

@@ -41,6 +41,12 @@ __global__ void __launch_bounds__(PRIMARY_THREADS) k_primary(const DeProgram* __
     float3 hp = mk3(0.f, 0.f, 0.f), grad = mk3(0.f, 0.f, 0.f);
     float hstep = 0.f, thit = 0.f;
     unsigned long long n_eval = 0, n_iter = 0, n_steps = 0;
+    auto store_normal = [&](float3 n) {
+        float* const q = pl.n + pix * pl.n_pixel;
+        q[0] = n.x;
+        q[pl.n_part] = n.y;
+        q[2 * pl.n_part] = n.z;
+    };
     // the ray's end: a hit at cand_t starts the normal taps, a miss writes its values
     auto end_ray = [&](bool hit) {
         pl.steps[pix] = m.i;
@@ -54,9 +60,7 @@ __global__ void __launch_bounds__(PRIMARY_THREADS) k_primary(const DeProgram* __
             state = PR_NORMAL;
         } else {
             pl.t[pix] = -1.0f;
-            pl.n[pix] = 0.f;
-            pl.n[total + pix] = 0.f;
-            pl.n[2 * total + pix] = 0.f;
+            store_normal(mk3(0.f, 0.f, 0.f));
             state = PR_IDLE;
         }
     };
@@ -102,9 +106,7 @@ __global__ void __launch_bounds__(PRIMARY_THREADS) k_primary(const DeProgram* __
                 if (++tap == taps) {
                     float3 n = normalize3(grad);
                     pl.t[pix] = thit;
-                    pl.n[pix] = n.x;
-                    pl.n[total + pix] = n.y;
-                    pl.n[2 * total + pix] = n.z;
+                    store_normal(n);
                     state = PR_IDLE;
                 }
             } else {

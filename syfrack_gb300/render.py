@@ -27,6 +27,11 @@ def _up(a):
     return a.ctypes.data_as(C.POINTER(C.c_uint32))
 
 
+# sf_de_sample as an array's records
+_SAMPLE = np.dtype([("distance", np.float32), ("traps", np.float32, 4), ("iterations", np.uint32),
+                    ("material", np.uint32)])
+
+
 @dataclass
 class DeSample:
     """crates/syfrack-core/src/scene/fractal.rs:18-27."""
@@ -126,16 +131,10 @@ class CompiledGraph:
         """Batched DE at points (n, 3) -> arrays distance, traps (n, 4), iterations, material."""
         pts = np.ascontiguousarray(points, dtype=np.float32).reshape(-1, 3)
         n = len(pts)
-        out = (abi.sf_de_sample * max(n, 1))()
-        check(self.ctx.lib.sf_de_probe(self.h, _fp(pts), n, out))
-        arr = np.ctypeslib.as_array(out)[:n] if n else np.zeros(0)
-        if n == 0:
-            return {"distance": np.zeros(0, np.float32), "traps": np.zeros((0, 4), np.float32),
-                    "iterations": np.zeros(0, np.uint32), "material": np.zeros(0, np.uint32)}
-        return {"distance": np.array([s.distance for s in out[:n]], dtype=np.float32),
-                "traps": np.array([list(s.traps) for s in out[:n]], dtype=np.float32),
-                "iterations": np.array([s.iterations for s in out[:n]], dtype=np.uint32),
-                "material": np.array([s.material for s in out[:n]], dtype=np.uint32)}
+        out = np.empty(n, _SAMPLE)
+        if n:
+            check(self.ctx.lib.sf_de_probe(self.h, _fp(pts), n, out.ctypes.data_as(C.POINTER(abi.sf_de_sample))))
+        return {k: np.ascontiguousarray(out[k]) for k in _SAMPLE.names}
 
 
 @dataclass
@@ -208,11 +207,11 @@ class Renderer:
         d.normal_mode = 0 if normal == "central" else 1
         d.eps, d.t_far, d.pixel_tolerance = eps, t_far, pixel_tolerance
         n = width * height
-        t = np.zeros(n, np.float32)
-        steps = np.zeros(n, np.uint32)
-        nrm = np.zeros((3, n), np.float32)
-        check(self.ctx.lib.sf_primary_trace(g.h, C.byref(d), _fp(t), _up(steps), _fp(nrm)))
-        return {"t": t, "steps": steps, "normal": nrm.T.copy()}
+        t = np.empty(n, np.float32)
+        steps = np.empty(n, np.uint32)
+        nrm = np.empty((n, 3), np.float32)
+        check(self.ctx.lib.sf_primary_trace_rows(g.h, C.byref(d), _fp(t), _up(steps), _fp(nrm)))
+        return {"t": t, "steps": steps, "normal": nrm}
 
 
 class RenderSession:
@@ -605,9 +604,9 @@ class Canvas:
 def escape2d(ctx: GpuContext, fractal: PlanarFractal, canvas: Canvas, tile=None, sample: int = 0xFFFFFFFF) -> dict:
     x, y, w, h = tile if tile else (0, 0, canvas.width, canvas.height)
     n = w * h
-    dist = np.zeros(n, np.float32)
-    traps = np.zeros((4, n), np.float32)
-    iters = np.zeros(n, np.uint32)
+    dist = np.empty(n, np.float32)
+    traps = np.empty((4, n), np.float32)
+    iters = np.empty(n, np.uint32)
     d, c = fractal.desc(), canvas.desc()
     check(ctx.lib.sf_escape2d(ctx.h, C.byref(d), C.byref(c), abi.sf_tile(x, y, w, h, 0), sample, _fp(dist),
                               _fp(traps), _up(iters)))
@@ -633,10 +632,10 @@ def deep_zoom(ctx: GpuContext, center_hi, center_lo, width_units: float, width: 
         keep = np.ascontiguousarray(given_orbit, dtype=np.float32).reshape(-1, 4)
         d.orbit_len, d.orbit = len(keep), _fp(keep)
     n = width * height
-    it = np.zeros(n, np.uint32)
-    sm = np.zeros(n, np.float32)
-    it64 = np.zeros(n if reference_f64 else 1, np.uint32)
-    sm64 = np.zeros(n if reference_f64 else 1, np.float32)
+    it = np.empty(n, np.uint32)
+    sm = np.empty(n, np.float32)
+    it64 = np.empty(n if reference_f64 else 1, np.uint32)
+    sm64 = np.empty(n if reference_f64 else 1, np.float32)
     reb = C.c_uint64()
     check(ctx.lib.sf_deep_zoom(ctx.h, C.byref(d), _up(it), _fp(sm), 1 if reference_f64 else 0, _up(it64),
                                _fp(sm64), C.byref(reb)))
