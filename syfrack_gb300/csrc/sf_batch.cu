@@ -3,7 +3,7 @@
 // path's job by binary search over the jobs' first paths. The job table is device
 // memory, so a captured CUDA graph can be replayed with advancing sample indices.
 #include "sf_stages.cuh"
-#include "sf_trace_kernel.cuh"
+#include "sf_batch_trace.cuh"
 
 static __device__ __forceinline__ void stage_begins(uint32_t* begins, const BatchTable& bt, bool pixels) {
     for (uint32_t i = threadIdx.x; i < bt.n_jobs; i += blockDim.x)
@@ -17,8 +17,10 @@ __global__ void __launch_bounds__(256) k_generate_batch(BatchTable bt, PathSoA s
     uint32_t path = blockIdx.x * blockDim.x + threadIdx.x;
     if (path == 0) {
         counts[0] = bt.total_paths;
-        counts[1] = bt.total_paths;
-        counts[2] = 0;
+        for (uint32_t g = 0; g < bt.groups; ++g) {
+            counts[1 + 2 * g] = bt.group_begin[g + 1] - bt.group_begin[g];
+            counts[2 + 2 * g] = 0;
+        }
     }
     if (path >= bt.total_paths) return;
     const BatchJob& job = bt.jobs[find_job(begins, bt.n_jobs, path)];
@@ -37,7 +39,15 @@ __global__ void __launch_bounds__(256) k_shade_batch(BatchTable bt, PathSoA soa,
         const BatchJob& job = bt.jobs[find_job(begins, bt.n_jobs, path)];
         uint32_t nf = shade_path<FEAT>(*job.scene, soa, job.geom, job.film, path - job.path_begin, path, status,
                                        final_round);
-        if (!final_round) enqueue_next(q, soa, nf, path);
+        if (final_round) continue;
+        enqueue_active(q, nf, path);
+        // group by group of the warp's lanes (one, but at the groups' borders)
+        const uint32_t lanes = __activemask();
+        for (uint32_t left = lanes; left != 0u;) {
+            const uint32_t g = __shfl_sync(lanes, job.group, __ffs(left) - 1);
+            if (job.group == g) enqueue_segments(q, soa, nf, path, g, bt.group_begin[g]);
+            left &= ~__ballot_sync(lanes, job.group == g);
+        }
     }
 }
 
@@ -81,25 +91,12 @@ cudaError_t sf_launch_advance_batch(BatchTable bt, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-template <int FORM>
-static cudaError_t launch_trace_batch_form(BatchTable bt, PathSoA soa, TraceLaunch tl, unsigned long long* stats,
-                                           int blocks, int min_blocks, cudaStream_t st) {
-    if (tl.optics) {  // a job with dielectric materials: the optics instantiation, 2 blocks per SM
-        k_trace<FORM, 2, true, false, true><<<blocks, 256, 0, st>>>(nullptr, nullptr, soa, tl, stats, bt);
-        return cudaGetLastError();
-    }
-    switch (min_blocks) {
-    case 3: k_trace<FORM, 3, true><<<blocks, 256, 0, st>>>(nullptr, nullptr, soa, tl, stats, bt); break;
-    case 4: k_trace<FORM, 4, true><<<blocks, 256, 0, st>>>(nullptr, nullptr, soa, tl, stats, bt); break;
-    default: k_trace<FORM, 2, true><<<blocks, 256, 0, st>>>(nullptr, nullptr, soa, tl, stats, bt); break;
-    }
-    return cudaGetLastError();
-}
-
 cudaError_t sf_launch_trace_batch(BatchTable bt, PathSoA soa, TraceLaunch tl, unsigned long long* stats, int blocks,
-                                  int min_blocks, int any_generic, cudaStream_t st) {
+                                  int min_blocks, cudaStream_t st) {
     if (min_blocks < 2 || min_blocks > 4) min_blocks = 2;
     if (blocks <= 0) blocks = sf_device_sm_count() * min_blocks;
-    if (any_generic) return launch_trace_batch_form<SF_FORM_ANY>(bt, soa, tl, stats, blocks, min_blocks, st);
-    return launch_trace_batch_form<SF_FORM_MIXED>(bt, soa, tl, stats, blocks, min_blocks, st);
+    for (uint32_t g = 0; g < bt.groups; ++g)
+        if (bt.group_form[g] == SF_FORM_GENERIC)
+            return sf_launch_trace_batch_generic(bt, soa, tl, stats, blocks, min_blocks, st);
+    return launch_trace_batch<false>(bt, soa, tl, stats, blocks, min_blocks, st);
 }

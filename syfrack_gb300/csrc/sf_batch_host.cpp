@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -16,7 +17,8 @@ using namespace sfh;
 struct sf_batch {
     sf_context* ctx = nullptr;
     std::vector<sf_graph*> graphs;
-    std::vector<BatchJob> jobs;  // host copy (initial sample_start)
+    std::vector<BatchJob> jobs;  // host copy (initial sample_start), sorted by group
+    std::vector<uint32_t> slot;  // the caller's job i is jobs[slot[i]]
     std::vector<sf_scene_desc> scenes;
     WaveArena a;
     cudaGraphExec_t exec = nullptr;
@@ -35,7 +37,8 @@ sf_status arena_alloc(sf_context* c, WaveArena& a, uint32_t capacity, uint32_t m
     size_t o_jobs = take(size_t(max_jobs) * sizeof(BatchJob));
     size_t o_Ls = take(N * 16), o_soa = take(wave_soa_bytes(N, K)), o_lists = take(wave_lists_bytes(N, K));
     size_t o_march = take(wave_march_bytes(N, K)), o_resume = take(wave_resume_bytes(N, K));
-    size_t o_counts = take(size_t(rounds + 1) * 16), o_qcounts = take(size_t(rounds) * 64 * 8), o_status = take(16);
+    size_t o_counts = take(wave_counts_bytes(rounds)), o_qcounts = take(wave_launch_counts_bytes(rounds));
+    size_t o_status = take(16);
     size_t o_extra = take(extra_bytes);
     sf_status st = ctx_alloc(c, off, &a.mem);
     if (st != SF_OK) return st;
@@ -56,13 +59,42 @@ sf_status arena_alloc(sf_context* c, WaveArena& a, uint32_t capacity, uint32_t m
     return SF_OK;
 }
 
+std::vector<uint32_t> group_keys(const std::vector<const sf_graph*>& graphs) {
+    std::vector<uint32_t> keys;
+    std::set<uint32_t> distinct;
+    for (const sf_graph* g : graphs) {
+        const FormParams& f = g->prog.fp;
+        const bool min0 = f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM;
+        uint32_t variant = 0;
+        if (g->prog.form == SF_FORM_BULB)
+            variant = !(min0 && f.trap_measure == SF_MEASURE_NORM) ? 2u : f.power_int == 8u ? 0u : 1u;
+        else if (g->prog.form == SF_FORM_BOX)
+            variant = (min0 && f.trap_squared ? 0u : 4u) | (f.fold_clamped ? 0u : 2u) | (f.scale < 0.0f ? 1u : 0u);
+        else if (g->prog.form == SF_FORM_MENGER)
+            variant = min0 && f.trap_squared ? 0u : 1u;
+        keys.push_back(g->prog.form * 8u + variant);
+        distinct.insert(keys.back());
+    }
+    if (distinct.size() > SF_MAX_GROUPS)
+        for (uint32_t& k : keys) k &= ~7u;
+    return keys;
+}
+uint32_t group_of(BatchTable& bt, uint32_t& last_key, uint32_t key, uint32_t form, uint32_t path_begin) {
+    if (bt.groups == 0 || last_key != key) {
+        bt.group_form[bt.groups] = form;
+        bt.group_begin[bt.groups++] = path_begin;
+    }
+    last_key = key;
+    return bt.groups - 1;
+}
+
 // One pass of a batched wavefront on stream st: every job of a.bt renders its samples.
 sf_status wave_record_pass(sf_context* c, const WaveArena& a, cudaStream_t st, bool timed) {
     const size_t N = a.capacity;
     const uint32_t R = a.rounds;
     const uint32_t Q = a.quantum ? std::min<uint32_t>((a.max_steps + a.quantum - 1) / a.quantum + 1, 64) : 1;
-    CU(cudaMemsetAsync(a.counts, 0, size_t(R + 1) * 16, st));
-    CU(cudaMemsetAsync(a.qcounts, 0, size_t(R) * 64 * 2 * 4, st));
+    CU(cudaMemsetAsync(a.counts, 0, wave_counts_bytes(R), st));
+    CU(cudaMemsetAsync(a.qcounts, 0, wave_launch_counts_bytes(R), st));
     {
         LaunchTimer t(c, false, timed, st);
         CU(sf_launch_generate_batch(a.bt, a.soa, a.counts, st));
@@ -75,19 +107,17 @@ sf_status wave_record_pass(sf_context* c, const WaveArena& a, cudaStream_t st, b
         for (uint32_t j = 0; j < Q; ++j) {
             TraceLaunch tl{};
             tl.q = q;
-            uint32_t* qc = a.qcounts + (size_t(r) * 64 + j) * 2;
-            tl.work_counter = qc;
+            tl.counts = wave_launch_counts(a.qcounts, r, j);
+            tl.last_counts = j == 0 ? nullptr : wave_launch_counts(a.qcounts, r, j - 1);
             tl.resume = j == 0 ? nullptr : wave_resume(a.resume, N, K, j - 1);
-            tl.resume_count = j == 0 ? nullptr : qc - 2 + 1;
             tl.next_resume = wave_resume(a.resume, N, K, j);
-            tl.next_resume_count = qc + 1;
             tl.quantum = j + 1 == Q ? 0u : a.quantum;
             tl.regen = a.regen;
             LaunchTimer t(c, true, timed, st);
             tl.optics = (a.rich & SF_RICH_OPTICS) ? 1u : 0u;
             // the optics trace kernel runs two blocks of 256 threads per SM
             CU(sf_launch_trace_batch(a.bt, a.soa, tl, c->d_stats, tl.optics ? 2 * c->sm_count : blocks,
-                                     int(a.min_blocks), a.any_generic ? 1 : 0, st));
+                                     int(a.min_blocks), st));
         }
         LaunchTimer t(c, false, timed, st);
         CU(sf_launch_shade_batch(a.bt, a.rich, a.soa, q, a.status, r + 1 == R ? 1 : 0, st));
@@ -132,7 +162,6 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
     if (n == 0 || n > SF_BATCH_MAX_JOBS) return fail(SF_ERR_INVALID, "a batch holds 1 to 1024 jobs");
     uint64_t paths = 0, pixels = 0, film_bytes = 0;
     uint32_t rounds = 0, max_steps = 0;
-    bool generic = false;
     for (uint32_t i = 0; i < n; ++i) {
         if (!jobs[i].graph || jobs[i].graph->ctx != c) return fail(SF_ERR_INVALID, "job graph missing or of another context");
         sf_status st = validate_config(jobs[i].cfg);
@@ -148,7 +177,6 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
         film_bytes += ((uint64_t(cf.width) * cf.height * (has_fog(jobs[i].scene) ? 84 : 36) + 255) & ~uint64_t(255));
         rounds = std::max(rounds, rounds_of(cf, jobs[i].scene));
         max_steps = std::max(max_steps, cf.max_steps);
-        generic |= jobs[i].graph->prog.form == SF_FORM_GENERIC;
     }
     if (paths > 0x7fffffffull) return fail(SF_ERR_INVALID, "batch too large (2^31 paths)");
     cudaSetDevice(c->device);
@@ -173,7 +201,6 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
                                scene_bytes + pv_bytes + ex_bytes + film_bytes, &extra);
     if (st != SF_OK) { delete b; return st; }
     b->a.max_steps = max_steps;
-    b->a.any_generic = generic;
     b->a.bt.n_jobs = n;
     b->a.bt.total_paths = uint32_t(paths);
     b->a.bt.total_pixels = uint32_t(pixels);
@@ -185,7 +212,15 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
     b->a.rich = rich;
     char* film = base + scene_bytes + pv_bytes + ex_bytes;
     uint32_t pbeg = 0, xbeg = 0;
-    for (uint32_t i = 0; i < n; ++i) {
+    std::vector<uint32_t> order(n);
+    for (uint32_t i = 0; i < n; ++i) order[i] = i;
+    std::vector<const sf_graph*> graphs;
+    for (uint32_t i = 0; i < n; ++i) graphs.push_back(jobs[i].graph);
+    const std::vector<uint32_t> keys = group_keys(graphs);
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return keys[x] < keys[y]; });
+    uint32_t last_key = 0;
+    b->slot.resize(n);
+    for (uint32_t i : order) {
         const sf_render_config& cf = jobs[i].cfg;
         uint32_t spd = std::max<uint32_t>(std::min(cf.samples_per_dispatch ? cf.samples_per_dispatch : cf.samples_per_pixel,
                                                    cf.samples_per_pixel), 1);
@@ -212,12 +247,15 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
         j.path_begin = pbeg;
         j.pixel_begin = xbeg;
         j.form = jobs[i].graph->prog.form;
+        j.group = group_of(b->a.bt, last_key, keys[i], j.form, pbeg);
         pbeg += uint32_t(px * spd);
         xbeg += uint32_t(px);
+        b->slot[i] = uint32_t(b->jobs.size());
         b->jobs.push_back(j);
         b->graphs.push_back(jobs[i].graph);
         graph_retain(jobs[i].graph);
     }
+    b->a.bt.group_begin[b->a.bt.groups] = pbeg;
     ctx_retain(c);
     cudaError_t e = cudaMemcpyAsync(d_scenes, scenes.data(), n * sizeof(DevScene), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) st = batch_reset(b);
@@ -341,7 +379,7 @@ extern "C" sf_status sf_batch_readback(sf_batch* b, uint32_t job, sf_film_planes
     if (job >= b->jobs.size()) return fail(SF_ERR_INVALID, "job index out of range");
     sf_context* c = b->ctx;
     cudaSetDevice(c->device);
-    CU(film_readback(c, b->jobs[job].film, *out, c->stream));
+    CU(film_readback(c, b->jobs[b->slot[job]].film, *out, c->stream));
     return SF_OK;
 }
 

@@ -1677,8 +1677,8 @@ sf_status session_alloc(sf_session* s) {
         o_march = take(wave_march_bytes(N, K));
         o_resume = take(wave_resume_bytes(N, K));
     }
-    size_t o_counts = take(size_t(R + 1) * 4 * 4);
-    size_t o_qcounts = take(size_t(R) * 64 * 2 * 4);
+    size_t o_counts = take(wave_counts_bytes(R));
+    size_t o_qcounts = take(wave_launch_counts_bytes(R));
     size_t o_status = take(16);
     s->mem_bytes = off;
     sf_status st = ctx_alloc(c, off, &s->mem);
@@ -1808,8 +1808,8 @@ extern "C" sf_status sf_session_dispatch(sf_session* s, sf_tile tile, uint32_t s
     const size_t N = s->capacity;
     // launches per round: the first, then one per step quantum a segment may still need
     const uint32_t Q = s->quantum ? std::min<uint32_t>((s->cfg.max_steps + s->quantum - 1) / s->quantum + 1, 64) : 1;
-    CU(cudaMemsetAsync(s->counts, 0, size_t(R + 1) * 16, st));
-    CU(cudaMemsetAsync(s->qcounts, 0, size_t(R) * 64 * 2 * 4, st));
+    CU(cudaMemsetAsync(s->counts, 0, wave_counts_bytes(R), st));
+    CU(cudaMemsetAsync(s->qcounts, 0, wave_launch_counts_bytes(R), st));
     {
         LaunchTimer t(c, false);
         CU(sf_launch_generate(s->d_scene, s->soa, g, s->counts, st));
@@ -1824,12 +1824,10 @@ extern "C" sf_status sf_session_dispatch(sf_session* s, sf_tile tile, uint32_t s
         for (uint32_t j = 0; j < Q; ++j) {
             TraceLaunch tl{};
             tl.q = q;
-            uint32_t* qc = s->qcounts + (size_t(r) * 64 + j) * 2;
-            tl.work_counter = qc;
+            tl.counts = wave_launch_counts(s->qcounts, r, j);
+            tl.last_counts = j == 0 ? nullptr : wave_launch_counts(s->qcounts, r, j - 1);
             tl.resume = j == 0 ? nullptr : wave_resume(s->resume, N, K, j - 1);
-            tl.resume_count = j == 0 ? nullptr : qc - 2 + 1;  // previous launch's resumed count
             tl.next_resume = wave_resume(s->resume, N, K, j);
-            tl.next_resume_count = qc + 1;
             tl.quantum = j + 1 == Q ? 0u : s->quantum;  // the last launch runs segments to completion
             tl.regen = s->regen;
             tl.lane_stats = c->lane_stats ? 1u : 0u;

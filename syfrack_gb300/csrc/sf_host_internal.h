@@ -222,12 +222,18 @@ inline void wave_round_queues(RoundQueues& q, uint32_t* lists, size_t N, uint32_
     q.active = r == 0 ? nullptr : cur;
     q.cont = r == 0 ? nullptr : cur + N;
     q.shadow = cur + 2 * N;
-    q.counts = counts + 4 * r;
+    q.counts = counts + SF_ROUND_COUNTS * r;
     q.next_active = nxt;
     q.next_cont = nxt + N;
     q.next_shadow = nxt + 2 * N;
-    q.next_counts = counts + 4 * (r + 1);
-    q.work_counter = counts + 4 * r + 3;
+    q.next_counts = counts + SF_ROUND_COUNTS * (r + 1);
+}
+// Counters of R rounds (and the one after) and of their launches, at most 64 a round.
+inline size_t wave_counts_bytes(uint32_t R) { return size_t(R + 1) * SF_ROUND_COUNTS * 4; }
+inline size_t wave_launch_counts_bytes(uint32_t R) { return size_t(R) * 64 * SF_LAUNCH_COUNTS * 4; }
+// Launch j of round r: its counters and resume lists.
+inline uint32_t* wave_launch_counts(uint32_t* qcounts, uint32_t r, uint32_t j) {
+    return qcounts + (size_t(r) * 64 + j) * SF_LAUNCH_COUNTS;
 }
 inline uint32_t* wave_resume(uint32_t* resume, size_t N, uint32_t K, uint32_t parity) {
     return resume + size_t(parity & 1) * (1 + size_t(K)) * N;
@@ -245,11 +251,19 @@ struct WaveArena {
     uint32_t* status = nullptr;
     void* mem = nullptr;
     size_t mem_bytes = 0;
-    bool any_generic = false;
     uint32_t rich = 0;  // SF_RICH_* of any job: the shading and trace kernels' features
     uint32_t min_blocks = 3, quantum = 128, regen = 4;
 };
 
+// The trace groups of a batch's jobs by their graphs: one key per job (jobs of one key
+// share a group; sort the table by it). A key is a form and the variant of its iteration
+// that the form's routine chooses, so that the lanes of a warp choose alike (a Mandelbox
+// pair of scales 2 and -2 took 8.3 instead of 6.6 ms with both in one group); with more
+// than SF_MAX_GROUPS of those, the form alone.
+std::vector<uint32_t> group_keys(const std::vector<const sf_graph*>& graphs);
+// Adds a job to the table being built, in key order: returns its group, which starts at
+// path_begin if the job opens it.
+uint32_t group_of(BatchTable& bt, uint32_t& last_key, uint32_t key, uint32_t form, uint32_t path_begin);
 sf_status arena_alloc(sf_context* c, WaveArena& a, uint32_t capacity, uint32_t max_jobs, uint32_t rounds,
                       uint32_t shadow_slots, size_t extra_bytes, size_t* extra_offset);
 sf_status wave_record_pass(sf_context* c, const WaveArena& a, cudaStream_t st, bool timed);
@@ -270,8 +284,8 @@ struct sf_session {
     uint32_t capacity = 0;
     uint32_t* lists = nullptr;     // 2 x {active, cont, shadow} x capacity
     uint32_t* resume = nullptr;    // 2 x 2*capacity segments cut at a step quantum
-    uint32_t* qcounts = nullptr;   // per round and launch: {work counter, resumed count}
-    uint32_t* counts = nullptr;    // per round: {active, cont, shadow, work}
+    uint32_t* qcounts = nullptr;   // per round and launch: SF_LAUNCH_COUNTS counters
+    uint32_t* counts = nullptr;    // per round: SF_ROUND_COUNTS counters
     uint32_t* status = nullptr;
     void* mem = nullptr;
     size_t mem_bytes = 0;

@@ -66,7 +66,9 @@ __global__ void __launch_bounds__(128, 5) k_shade(const DevScene* __restrict__ s
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         uint32_t path = q.active ? q.active[j] : j;
         uint32_t nf = shade_path<FEAT>(S, soa, g, film, path, path, status, final_round);
-        if (!final_round) enqueue_next(q, soa, nf, path);
+        if (final_round) continue;
+        enqueue_active(q, nf, path);
+        enqueue_segments(q, soa, nf, path, 0, 0);
     }
 }
 

@@ -54,31 +54,39 @@ struct PathSoA {
     uint32_t shadow_slots;  // K: sh_o/sh_d/sh_c/vis have K * capacity rows (row = k * capacity + path)
 };
 
-// Queues of one round: active paths, continuation rays, shadow rays (ids),
-// with their counts in `counts[0..2]`; next round's lists are written by shade.
+// Counters of a round: active paths, then per group of jobs its continuation and its
+// shadow segments (a session is one group, a batch one per form and variant of it).
+#define SF_MAX_GROUPS 8
+#define SF_ROUND_COUNTS (1 + 2 * SF_MAX_GROUPS)
+// Counters of one trace launch: per group {work counter, resumed segments}.
+#define SF_LAUNCH_COUNTS (2 * SF_MAX_GROUPS)
+
+// Queues of one round: active paths, continuation rays, shadow rays (ids), with their
+// SF_ROUND_COUNTS counters; next round's lists are written by shade. A group whose
+// paths start at b has its continuations at cont + b and its shadow rows at
+// shadow + shadow_slots * b.
 struct RoundQueues {
     const uint32_t* active;   // null: identity (round 0)
     const uint32_t* cont;     // null: identity (round 0)
     const uint32_t* shadow;
-    const uint32_t* counts;   // [active, cont, shadow]
+    const uint32_t* counts;
     uint32_t* next_active;
     uint32_t* next_cont;
     uint32_t* next_shadow;
-    uint32_t* next_counts;    // [active, cont, shadow]
-    uint32_t* work_counter;   // trace kernel fetch counter (zeroed per round)
+    uint32_t* next_counts;
 };
 
 // One launch of the persistent trace kernel: the round's fresh segments
 // (continuations then shadows) or the segments resumed after a step quantum.
 // Item encoding: continuation lists hold paths, shadow lists shadow rows
 // (k * capacity + path); resume lists hold path or shadow row | (shadow ? 1u << 31 : 0).
+// A group's resumed segments are at (1 + shadow_slots) * its first path.
 struct TraceLaunch {
     RoundQueues q;
     const uint32_t* resume;       // null on the first launch of a round
-    const uint32_t* resume_count;
     uint32_t* next_resume;        // segments cut at this launch's quantum
-    uint32_t* next_resume_count;
-    uint32_t* work_counter;
+    const uint32_t* last_counts;  // the round's previous launch's SF_LAUNCH_COUNTS counters
+    uint32_t* counts;             // this launch's, zero at its start
     uint32_t quantum;             // march steps per segment per launch (0 = unbounded)
     uint32_t regen;               // idle lanes a warp waits for before it takes new segments (1..32)
     uint32_t lane_stats;          // 1: count warp-level DE calls and iteration slots (diagnostic kernel)
@@ -154,15 +162,19 @@ struct BatchJob {
     uint32_t path_begin;
     uint32_t pixel_begin;
     uint32_t form;
-    uint32_t pad;
+    uint32_t group;  // of BatchTable
 };
 #define SF_BATCH_MAX_JOBS 1024
+// The jobs are sorted by group: group g holds jobs of form group_form[g], whose paths are
+// [group_begin[g], group_begin[g + 1]).
 struct BatchTable {
     BatchJob* jobs;
     uint32_t n_jobs;
     uint32_t total_paths;
     uint32_t total_pixels;
-    uint32_t pad;
+    uint32_t groups;
+    uint32_t group_form[SF_MAX_GROUPS];
+    uint32_t group_begin[SF_MAX_GROUPS + 1];
 };
 
 // ---- launchers (return cudaError_t of the launch) ----
@@ -199,7 +211,10 @@ cudaError_t sf_launch_trace_any(const DeProgram*, const DevScene*, PathSoA, Trac
 // Batched wavefront (sf_batch.cu): all jobs' paths in one set of launches.
 cudaError_t sf_launch_generate_batch(BatchTable bt, PathSoA soa, uint32_t* counts, cudaStream_t st);
 cudaError_t sf_launch_trace_batch(BatchTable bt, PathSoA soa, TraceLaunch tl, unsigned long long* stats, int blocks,
-                                  int min_blocks, int any_generic, cudaStream_t st);
+                                  int min_blocks, cudaStream_t st);
+// The same with a group of generic graphs among the batch's (sf_batch_generic.cu).
+cudaError_t sf_launch_trace_batch_generic(BatchTable bt, PathSoA soa, TraceLaunch tl, unsigned long long* stats,
+                                          int blocks, int min_blocks, cudaStream_t st);
 cudaError_t sf_launch_shade_batch(BatchTable bt, uint32_t rich, PathSoA soa, RoundQueues q, uint32_t* status, int final_round,
                                   cudaStream_t st);
 cudaError_t sf_launch_commit_batch(BatchTable bt, PathSoA soa, cudaStream_t st);

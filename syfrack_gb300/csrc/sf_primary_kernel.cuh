@@ -91,12 +91,12 @@ __global__ void __launch_bounds__(PRIMARY_THREADS) k_primary(const DeProgram* __
             const float3 qp = state == PR_NORMAL
                                   ? hp + (normal_mode == 0 ? central_offset(tap) : tetra_offset(tap)) * hstep
                                   : m.ro + m.rd * m.t;
-            DeRaw s = de_form<FORM>(P, qp);
+            DeRaw s = de_form<FORM>(P, P.fp, qp);
             n_eval++;
             n_iter += s.iter;
             if constexpr (FORM == SF_FORM_ANY) {
                 if (state == PR_MARCH && needs_exact(s, m.t, S.step_scale, accept, absolute)) {
-                    s = de_raw_exact(P, qp);
+                    s = de_form_exact<FORM>(P, P.fp, qp);
                     n_eval++;
                     n_iter += s.iter;
                 }

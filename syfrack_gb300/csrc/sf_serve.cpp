@@ -319,8 +319,17 @@ sf_status launch_wave(sf_server* s, ServeSlot& sl) {
     BatchJob* hj = reinterpret_cast<BatchJob*>(sl.stage + stage_jobs_off(s));
     DevScene* hs = reinterpret_cast<DevScene*>(sl.stage + stage_scenes_off(s));
     uint32_t paths = 0, pixels = 0, rounds = 0, steps = 0, n_scenes = 0, rich = 0;
-    for (size_t i = 0; i < sl.reqs.size(); ++i) {
-        ServeReq* r = sl.reqs[i];
+    // the job table sorted by group (the requests keep their order: a film's passes)
+    std::vector<const sf_graph*> graphs;
+    for (const ServeReq* r : sl.reqs) graphs.push_back(r->film->graph);
+    const std::vector<uint32_t> keys = group_keys(graphs);
+    std::vector<uint32_t> order(sl.reqs.size());
+    for (uint32_t i = 0; i < order.size(); ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return keys[x] < keys[y]; });
+    uint32_t last_key = 0;
+    a.bt.groups = 0;
+    for (size_t i = 0; i < order.size(); ++i) {
+        ServeReq* r = sl.reqs[order[i]];
         ServeFilm* f = r->film;
         uint32_t px = r->width * r->height;
         BatchJob j{};
@@ -331,6 +340,7 @@ sf_status launch_wave(sf_server* s, ServeSlot& sl) {
         j.path_begin = paths;
         j.pixel_begin = pixels;
         j.form = f->graph->prog.form;
+        j.group = group_of(a.bt, last_key, keys[order[i]], j.form, paths);
         hj[i] = j;
         paths += px * r->samples;
         pixels += px;
@@ -348,9 +358,9 @@ sf_status launch_wave(sf_server* s, ServeSlot& sl) {
     }
     a.bt.n_jobs = uint32_t(sl.reqs.size());
     a.bt.total_paths = paths;
+    a.bt.group_begin[a.bt.groups] = paths;
     a.bt.total_pixels = pixels;
     a.max_steps = steps;
-    a.any_generic = sl.cls == SC_GENERIC;
     CU(cudaMemcpyAsync(a.bt.jobs, hj, sl.reqs.size() * sizeof(BatchJob), cudaMemcpyHostToDevice, st));
     CU(cudaMemsetAsync(a.status, 0, 16, st));
     // rounds vary per batch; the arena's queue counters are sized for its largest

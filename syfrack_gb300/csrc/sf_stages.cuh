@@ -197,13 +197,17 @@ static __device__ __forceinline__ uint32_t shade_path(const DevScene& S, PathSoA
     return nf;
 }
 
-static __device__ __forceinline__ void enqueue_next(const RoundQueues& q, const PathSoA& soa, uint32_t nf,
-                                                    uint32_t path) {
+static __device__ __forceinline__ void enqueue_active(const RoundQueues& q, uint32_t nf, uint32_t path) {
     warp_append(&q.next_counts[0], q.next_active, nf != 0, path);
-    warp_append(&q.next_counts[1], q.next_cont, (nf & SF_PF_CONT) != 0, path);
+}
+// The path's segments into the lists of its group, whose paths start at first_path.
+static __device__ __forceinline__ void enqueue_segments(const RoundQueues& q, const PathSoA& soa, uint32_t nf,
+                                                        uint32_t path, uint32_t group, uint32_t first_path) {
+    warp_append(&q.next_counts[1 + 2 * group], q.next_cont + first_path, (nf & SF_PF_CONT) != 0, path);
     const uint32_t mask = (nf & SF_PF_SHADOW) ? (nf >> SF_PF_SHADOW_SHIFT) & 0xffu : 0u;
+    uint32_t* const shadow = q.next_shadow + size_t(soa.shadow_slots) * first_path;
     for (uint32_t k = 0; k < soa.shadow_slots; ++k)
-        warp_append(&q.next_counts[2], q.next_shadow, ((mask >> k) & 1u) != 0, k * soa.capacity + path);
+        warp_append(&q.next_counts[2 + 2 * group], shadow, ((mask >> k) & 1u) != 0, k * soa.capacity + path);
 }
 
 // wf_commit (wavefront.wgsl:232-260) for one pixel: ordered per-sample film add in

@@ -16,8 +16,7 @@
 #include "sf_warp.cuh"
 
 enum { TL_IDLE = 0, TL_MARCH = 1, TL_CAND = 2, TL_NORMAL = 3, TL_DONE = 4, TL_INIT = 5, TL_REFINE = 6, TL_FINAL = 7 };
-#define SF_FORM_ANY 99u
-#define SF_FORM_MIXED 98u  // any of the three iterated forms, chosen per lane
+#define SF_FORM_ANY 99u  // the generic interpreter
 
 // fp: the form's constants, P's own or those of the launch (TraceLaunch.fp).
 template <int FORM>
@@ -25,20 +24,12 @@ __device__ __forceinline__ DeRaw de_form(const DeProgram& P, const FormParams& f
     if constexpr (FORM == SF_FORM_BULB) return de_bulb(fp, p);
     else if constexpr (FORM == SF_FORM_BOX) return de_box(fp, p);
     else if constexpr (FORM == SF_FORM_MENGER) return de_menger(fp, p);
-    else return de_raw(P, p);
+    else return de_generic(P, p, false);
 }
 template <int FORM>
-__device__ __forceinline__ DeRaw de_form(const DeProgram& P, float3 p) {
-    if constexpr (FORM == SF_FORM_BULB) return de_bulb(P.fp, p);
-    else if constexpr (FORM == SF_FORM_BOX) return de_box(P.fp, p);
-    else if constexpr (FORM == SF_FORM_MENGER) return de_menger(P.fp, p);
-    else if constexpr (FORM == SF_FORM_MIXED) {
-        switch (P.form) {
-        case SF_FORM_BULB: return de_bulb(P.fp, p);
-        case SF_FORM_BOX: return de_box(P.fp, p);
-        default: return de_menger(P.fp, p);
-        }
-    } else return de_raw(P, p);
+__device__ __forceinline__ DeRaw de_form_exact(const DeProgram& P, const FormParams& fp, float3 p) {
+    if constexpr (FORM == SF_FORM_ANY) return de_generic(P, p, true);
+    else return de_form<FORM>(P, fp, p);
 }
 
 // Job of a batched path: binary search of the jobs' first paths (staged in shared memory).
@@ -52,6 +43,13 @@ static __device__ __forceinline__ uint32_t find_job(const uint32_t* begins, uint
     return lo;
 }
 
+// One group of a launch's work items, all of one form (a session's only group, or the
+// jobs of one form of a batch).
+struct TraceGroup {
+    uint32_t index;       // its counters
+    uint32_t first_path;  // where its paths start
+};
+
 // MULTI: the work items belong to the jobs of a batch (bt); each lane reads its job's
 // program and scene (L1-cached global memory) when it takes an item.
 // LANE_STATS: also count warp-level DE calls and, per call, the warp's longest
@@ -63,27 +61,14 @@ static __device__ __forceinline__ uint32_t find_job(const uint32_t* begins, uint
 // 1e-4; a shadow segment crosses such surfaces, its weight (PathSoA.sh_d.w) times
 // 1 - opacity at each, and marches on from just past them, up to 32 crossings
 // (geometry_visibility_weight, lights.wgsl:263-283).
-// THREADS: 256, or 128 for the shapes that fit more warps per SM at the same registers.
-template <int FORM, int MIN_BLOCKS, bool MULTI = false, bool LANE_STATS = false, bool OPTICS = false,
-          int THREADS = 256>
-__global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* __restrict__ prog_g,
-                                                           const DevScene* __restrict__ scene_g, PathSoA soa,
-                                                           TraceLaunch tl, unsigned long long* stats,
-                                                           BatchTable bt = BatchTable{}) {
-    __shared__ DeProgram P;
-    __shared__ DevScene S;
-    __shared__ uint32_t begins[MULTI ? SF_BATCH_MAX_JOBS : 1];
-    if constexpr (MULTI) {
-        for (uint32_t i = threadIdx.x; i < bt.n_jobs; i += blockDim.x) begins[i] = bt.jobs[i].path_begin;
-    } else {
-        stage_program(P, prog_g);
-        stage_pod(S, scene_g);
-        stage_more_lights(scene_g);
-    }
-    __syncthreads();
+template <int FORM, bool MULTI, bool LANE_STATS, bool OPTICS>
+__device__ __forceinline__ void trace_group(const DeProgram& P, const DevScene& S, const uint32_t* begins, PathSoA& soa,
+                                            const TraceLaunch& tl, unsigned long long* stats, const BatchTable& bt,
+                                            TraceGroup group) {
     const bool first = tl.resume == nullptr;
-    const uint32_t n_cont = first ? tl.q.counts[1] : 0u;
-    const uint32_t total = first ? n_cont + tl.q.counts[2] : *tl.resume_count;
+    const uint32_t n_cont = first ? tl.q.counts[1 + 2 * group.index] : 0u;
+    const uint32_t total = first ? n_cont + tl.q.counts[2 + 2 * group.index] : tl.last_counts[2 * group.index + 1];
+    uint32_t* const work_counter = tl.counts + 2 * group.index;
     const uint32_t quantum = tl.quantum ? tl.quantum : 0xffffffffu;
     const DeProgram* Pl = &P;
     const DevScene* Sl = &S;
@@ -185,7 +170,7 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* 
         const uint32_t idle = quiet ? __ballot_sync(FULL_MASK, state == TL_IDLE) : 0u;  // warp-uniform
         if (quiet == FULL_MASK && idle == 0u) break;  // every lane done
         if (idle && ((uint32_t)__popc(idle) >= regen || quiet == FULL_MASK)) {  // warp-uniform
-            const uint32_t w = warp_fetch(tl.work_counter, state == TL_IDLE);
+            const uint32_t w = warp_fetch(work_counter, state == TL_IDLE);
             if constexpr (LANE_STATS) {
                 if (t_dry == 0 && __any_sync(FULL_MASK, state == TL_IDLE && w >= total)) t_dry = clock64();
             }
@@ -195,9 +180,10 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* 
                 } else {
                     if (first) {
                         shadow = w >= n_cont;
-                        item = shadow ? tl.q.shadow[w - n_cont] : (tl.q.cont ? tl.q.cont[w] : w);
+                        item = shadow ? tl.q.shadow[size_t(soa.shadow_slots) * group.first_path + (w - n_cont)]
+                                      : (tl.q.cont ? tl.q.cont[group.first_path + w] : group.first_path + w);
                     } else {
-                        const uint32_t it = tl.resume[w];
+                        const uint32_t it = tl.resume[(1 + size_t(soa.shadow_slots)) * group.first_path + w];
                         item = it & 0x7fffffffu;
                         shadow = (it >> 31) != 0;
                     }
@@ -239,18 +225,16 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* 
             // the single-job kernel reads the program from shared memory by name (LDS)
             DeRaw s;
             const bool exact_state = OPTICS && (state == TL_INIT || state == TL_REFINE || state == TL_FINAL);
-            if constexpr (MULTI && FORM == SF_FORM_ANY && OPTICS)
-                s = exact_state ? de_raw_exact(*Pl, q) : de_form<FORM>(*Pl, q);
-            else if constexpr (MULTI) s = de_form<FORM>(*Pl, q);
-            else if constexpr (FORM == SF_FORM_ANY && OPTICS) s = exact_state ? de_raw_exact(P, q) : de_form<FORM>(P, q);
-            else s = de_form<FORM>(P, tl.fp, q);
+            const DeProgram& Pq = MULTI ? *Pl : P;
+            const FormParams& fq = MULTI ? Pl->fp : tl.fp;
+            if (OPTICS && FORM == SF_FORM_ANY && exact_state) s = de_form_exact<FORM>(Pq, fq, q);
+            else s = de_form<FORM>(Pq, fq, q);
             n_eval++;
             n_iter += s.iter;
             if constexpr (FORM == SF_FORM_ANY) {
                 // a flagged march or candidate sample near acceptance: the exact sample
                 if (state != TL_NORMAL && !exact_state && needs_exact(s, m.t, TR_SAFETY, TR_ACCEPT, TR_ABSOLUTE)) {
-                    if constexpr (MULTI) s = de_raw_exact(*Pl, q);
-                    else s = de_raw_exact(P, q);
+                    s = de_form_exact<FORM>(Pq, fq, q);
                     n_eval++;
                     n_iter += s.iter;
                 }
@@ -368,7 +352,9 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* 
                         soa.m0[row] = make_float4(m.t, m.omega, m.prev_radius, m.step_len);
                         soa.m1[row] = make_float4(m.t_end, m.cand_t, m.cand_err, __uint_as_float(m.i));
                         soa.m2[row] = li;
-                        warp_append(tl.next_resume_count, tl.next_resume, true, item | (shadow ? 0x80000000u : 0u));
+                        warp_append(work_counter + 1,
+                                    tl.next_resume + (1 + size_t(soa.shadow_slots)) * group.first_path, true,
+                                    item | (shadow ? 0x80000000u : 0u));
                         state = TL_IDLE;
                     }
                 }
@@ -394,27 +380,42 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* 
 #undef TR_TOL
 }
 
+// One job's segments, all of one form. THREADS: 256, or 128 for the shapes that fit more
+// warps per SM at the same registers.
+template <int FORM, int MIN_BLOCKS, bool LANE_STATS = false, bool OPTICS = false, int THREADS = 256>
+__global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_trace(const DeProgram* __restrict__ prog_g,
+                                                           const DevScene* __restrict__ scene_g, PathSoA soa,
+                                                           TraceLaunch tl, unsigned long long* stats) {
+    __shared__ DeProgram P;
+    __shared__ DevScene S;
+    stage_program(P, prog_g);
+    stage_pod(S, scene_g);
+    stage_more_lights(scene_g);
+    __syncthreads();
+    trace_group<FORM, false, LANE_STATS, OPTICS>(P, S, nullptr, soa, tl, stats, BatchTable{}, TraceGroup{0, 0});
+}
+
 template <int FORM>
 static cudaError_t launch_trace_form(const DeProgram* prog, const DevScene* scene, PathSoA soa, TraceLaunch tl,
                                      unsigned long long* stats, int blocks, int min_blocks, uint32_t light_smem, cudaStream_t st) {
     if (tl.optics) {  // 6 blocks of 128 threads per SM (the host sizes the grid)
-        k_trace<FORM, 6, false, false, true, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats);
+        k_trace<FORM, 6, false, true, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats);
         return cudaGetLastError();
     }
     if (tl.lane_stats && min_blocks == 3) {
-        k_trace<FORM, 3, false, true><<<blocks, 256, light_smem, st>>>(prog, scene, soa, tl, stats);
+        k_trace<FORM, 3, true><<<blocks, 256, light_smem, st>>>(prog, scene, soa, tl, stats);
         return cudaGetLastError();
     }
     if (tl.lane_stats && min_blocks == 7) {
-        k_trace<FORM, 7, false, true, false, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats);
+        k_trace<FORM, 7, true, false, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats);
         return cudaGetLastError();
     }
     switch (min_blocks) {
     case 3: k_trace<FORM, 3><<<blocks, 256, light_smem, st>>>(prog, scene, soa, tl, stats); break;
     case 4: k_trace<FORM, 4><<<blocks, 256, light_smem, st>>>(prog, scene, soa, tl, stats); break;
     // 128-thread blocks: 6 or 7 per SM (24 or 28 warps at up to 85 or 73 registers)
-    case 6: k_trace<FORM, 6, false, false, false, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats); break;
-    case 7: k_trace<FORM, 7, false, false, false, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats); break;
+    case 6: k_trace<FORM, 6, false, false, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats); break;
+    case 7: k_trace<FORM, 7, false, false, 128><<<blocks, 128, light_smem, st>>>(prog, scene, soa, tl, stats); break;
     default: k_trace<FORM, 2><<<blocks, 256, light_smem, st>>>(prog, scene, soa, tl, stats); break;
     }
     return cudaGetLastError();
