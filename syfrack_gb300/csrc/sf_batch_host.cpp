@@ -67,9 +67,9 @@ std::vector<uint32_t> group_keys(const std::vector<const sf_graph*>& graphs) {
         const bool min0 = f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM;
         uint32_t variant = 0;
         if (g->prog.form == SF_FORM_BULB)
-            variant = !(min0 && f.trap_measure == SF_MEASURE_NORM) ? 2u : f.power_int == 8u ? 0u : 1u;
+            variant = min0 && f.trap_measure == SF_MEASURE_NORM ? 0u : 1u;
         else if (g->prog.form == SF_FORM_BOX)
-            variant = (min0 && f.trap_squared ? 0u : 4u) | (f.fold_clamped ? 0u : 2u) | (f.scale < 0.0f ? 1u : 0u);
+            variant = (min0 && f.trap_squared ? 0u : 2u) | (f.fold_clamped ? 0u : 1u);
         else if (g->prog.form == SF_FORM_MENGER)
             variant = min0 && f.trap_squared ? 0u : 1u;
         keys.push_back(g->prog.form * 8u + variant);
@@ -201,6 +201,11 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
                                scene_bytes + pv_bytes + ex_bytes + film_bytes, &extra);
     if (st != SF_OK) { delete b; return st; }
     b->a.max_steps = max_steps;
+    // until set_launch or autotune: over 4, 10, 16 and 64 mixed jobs 9.0, 7.6, 9.3 and 60 ms
+    // a pass, against 10.4, 8.8, 11.4 and 67 at 3 blocks, quantum 128, regeneration 4
+    b->a.min_blocks = 4;
+    b->a.quantum = 0;
+    b->a.regen = 8;
     b->a.bt.n_jobs = n;
     b->a.bt.total_paths = uint32_t(paths);
     b->a.bt.total_pixels = uint32_t(pixels);

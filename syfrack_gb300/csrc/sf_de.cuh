@@ -296,9 +296,11 @@ __device__ __forceinline__ DeRaw de_bulb_t(const FormParams& f, float3 p) {
     s.material = f.material;
     return s;
 }
+// BATCH: one routine for every power and scale, so that lanes of different jobs keep together.
+template <bool BATCH = false>
 __device__ __forceinline__ DeRaw de_bulb(const FormParams& f, float3 p) {
     if (f.trap_measure == SF_MEASURE_NORM && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM)
-        return f.power_int == 8u ? de_bulb_t<true, 8u>(f, p) : de_bulb_t<true, 0u>(f, p);
+        return !BATCH && f.power_int == 8u ? de_bulb_t<true, 8u>(f, p) : de_bulb_t<true, 0u>(f, p);
     return de_bulb_t<false, 0u>(f, p);
 }
 
@@ -345,6 +347,11 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     F2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
@@ -358,10 +365,11 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 // reference's three cases (eval.rs:408-414) are min(fr^2/mr^2, max(fr^2/r^2, 1)),
 // two min/max instead of a compare and a select; otherwise the factor for
 // r^2 >= min_radius^2 is max(fr^2 / r^2, 1), which covers r^2 >= fixed_radius^2.
-// NEG (scale < 0): the sign that turns the point's factor -k * scale into the
-// derivative's k * |scale| is known, so one packed product serves the three components
-// and dr (with two products the launch took 122.7 instead of 119.0 ms per 64-spp frame).
-template <bool NORM_MIN0, bool CLAMPED, bool NEG>
+// SIGN: that of the scale, which turns the point's factor -k * scale into the
+// derivative's k * |scale|, so one packed product serves the three components and dr;
+// 0 when it is not known, with two products (the launch took 122.7 instead of 119.0 ms
+// per 64-spp frame).
+template <bool NORM_MIN0, bool CLAMPED, int SIGN>
 __device__ __forceinline__ DeRaw de_box_t(const FormParams& f, float3 p) {
     DeRaw s = raw_empty();
     float dr = 1.0f;
@@ -374,7 +382,7 @@ __device__ __forceinline__ DeRaw de_box_t(const FormParams& f, float3 p) {
     // fold * (-k scale) + (-c). Every result is the exact negation of the same
     // operation on p, so the iteration rounds as it does on p.
     const float ncx = -p.x, ncy = -p.y, ncz = -p.z;
-    const F2 ncxy = pack2(ncx, ncy), nsc = dup2(-f.scale);
+    const F2 ncxy = pack2(ncx, ncy), nsc = SIGN ? dup2(-f.scale) : pack2(-f.scale, fabsf(f.scale));
     float wx = ncx, wy = ncy, wz = ncz;
     uint32_t i = 0;
 #pragma unroll 2
@@ -393,13 +401,13 @@ __device__ __forceinline__ DeRaw de_box_t(const FormParams& f, float3 p) {
         const float qk = fr2 * rcp_approx(r2);
         const float k = CLAMPED ? fminf(kmin, fmaxf(qk, 1.0f)) : (r2 < mr2 ? kmin : fmaxf(qk, 1.0f));
         // sphere fold, Scale and AddOrigin as one multiply-add per component
-        const F2 kx = mul2(dup2(k), nsc);  // -k * scale, twice
-        const float2 wxy = unpack2(fma2(pack2(q.x, q.y), kx, ncxy));
+        const F2 kk = mul2(dup2(k), nsc);  // -k * scale twice, or beside k * |scale|
+        const float2 ks = unpack2(kk);
+        const float2 wxy = unpack2(fma2(pack2(q.x, q.y), SIGN ? kk : dup2(ks.x), ncxy));
         wx = wxy.x;
         wy = wxy.y;
-        const float kz = unpack2(kx).x;
-        wz = fmaf(q.z, kz, ncz);
-        dr = fmaf(dr, NEG ? kz : -kz, 1.0f);  // k * |scale|
+        wz = fmaf(q.z, ks.x, ncz);
+        dr = fmaf(dr, SIGN == 0 ? ks.y : SIGN < 0 ? ks.x : -ks.x, 1.0f);
     }
     s.iter = i;
     s.d = (sqrt_fast(fmaf(wz, wz, fmaf(wx, wx, wy * wy))) - f.fence[0]) * rcp_approx(fabsf(dr));
@@ -408,15 +416,16 @@ __device__ __forceinline__ DeRaw de_box_t(const FormParams& f, float3 p) {
     else if (sq) trap_sqrt(s, f.trap_slot);
     return s;
 }
-template <bool NORM_MIN0>
-__device__ __forceinline__ DeRaw de_box_n(const FormParams& f, float3 p) {
-    if (f.fold_clamped)
-        return f.scale < 0.0f ? de_box_t<NORM_MIN0, true, true>(f, p) : de_box_t<NORM_MIN0, true, false>(f, p);
-    return f.scale < 0.0f ? de_box_t<NORM_MIN0, false, true>(f, p) : de_box_t<NORM_MIN0, false, false>(f, p);
+template <bool NORM_MIN0, bool CLAMPED, bool BATCH>
+__device__ __forceinline__ DeRaw de_box_c(const FormParams& f, float3 p) {
+    if (BATCH) return de_box_t<NORM_MIN0, CLAMPED, 0>(f, p);
+    return f.scale < 0.0f ? de_box_t<NORM_MIN0, CLAMPED, -1>(f, p) : de_box_t<NORM_MIN0, CLAMPED, 1>(f, p);
 }
+template <bool BATCH = false>
 __device__ __forceinline__ DeRaw de_box(const FormParams& f, float3 p) {
-    if (f.trap_squared && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM) return de_box_n<true>(f, p);
-    return de_box_n<false>(f, p);
+    if (f.trap_squared && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM)
+        return f.fold_clamped ? de_box_c<true, true, BATCH>(f, p) : de_box_c<true, false, BATCH>(f, p);
+    return f.fold_clamped ? de_box_c<false, true, BATCH>(f, p) : de_box_c<false, false, BATCH>(f, p);
 }
 
 // Menger: Iterate{MengerFold, Trap} -> Box (graphs/menger.ron).
@@ -1079,8 +1088,8 @@ static __device__ __noinline__ DeRaw de_union_exact(const DeProgram& P, float3 c
 // Entry point: raw DE at p for the program's form.
 __device__ __forceinline__ DeRaw de_raw(const DeProgram& P, float3 p) {
     switch (P.form) {
-    case SF_FORM_BULB: return de_bulb(P.fp, p);
-    case SF_FORM_BOX: return de_box(P.fp, p);
+    case SF_FORM_BULB: return de_bulb<>(P.fp, p);
+    case SF_FORM_BOX: return de_box<>(P.fp, p);
     case SF_FORM_MENGER: return de_menger(P.fp, p);
     default: return de_generic(P, p, false);
     }

@@ -257,9 +257,10 @@ struct WaveArena {
 
 // The trace groups of a batch's jobs by their graphs: one key per job (jobs of one key
 // share a group; sort the table by it). A key is a form and the variant of its iteration
-// that the form's routine chooses, so that the lanes of a warp choose alike (a Mandelbox
-// pair of scales 2 and -2 took 8.3 instead of 6.6 ms with both in one group); with more
-// than SF_MAX_GROUPS of those, the form alone.
+// that the form's routine chooses (the trap, the fold's clamp), so that the lanes of a
+// warp choose alike; with more than SF_MAX_GROUPS of those, the form alone. Every group
+// costs its warps a wait for their longest segments, so what a batch can run in one
+// routine stays in one group: a Mandelbox pair of scales 2 and -2 took 7.1 ms as two.
 std::vector<uint32_t> group_keys(const std::vector<const sf_graph*>& graphs);
 // Adds a job to the table being built, in key order: returns its group, which starts at
 // path_begin if the job opens it.

@@ -435,19 +435,16 @@ static __device__ __forceinline__ OrbitQuad load_quad(const float2* p) {  // 32-
     return r;
 }
 
-// One iteration of a pixel's offset d = (dx, dy) from Z_m = z0 to Z_(m+1) = z1: the new
-// point (zx, zy), its |z|^2 and the offset's |d|^2.
-static __device__ __forceinline__ void pert_step(float2 z0, float2 z1, float dcx, float dcy, float& dx, float& dy,
-                                                 float& zx, float& zy, float& mag, float& dd) {
-    const float tx = fmaf(2.0f, z0.x, dx), ty = fmaf(2.0f, z0.y, dy);
-    const float ndx = __fadd_rn(diff_of_products(tx, dx, ty, dy), dcx);
-    const float ndy = __fadd_rn(sum_of_products(tx, dy, ty, dx), dcy);
-    dx = ndx;
-    dy = ndy;
-    zx = __fadd_rn(z1.x, dx);
-    zy = __fadd_rn(z1.y, dy);
-    mag = sum_of_products(zx, zx, zy, zy);
-    dd = sum_of_products(dx, dx, dy, dy);
+// One iteration of a pixel's offset d from Z_m = z0 to Z_(m+1) = z1: the new point z, its
+// |z|^2 and the offset's |d|^2. The sums of pairs are packed (each half rounds as a
+// binary32 operation): 40.9 -> 36.7 ms.
+static __device__ __forceinline__ void pert_step(float2 z0, float2 z1, F2 dc, F2& d, float2& z, float& mag, float& dd) {
+    const float2 v = unpack2(d), t = unpack2(fma2(dup2(2.0f), pack2(z0.x, z0.y), d));
+    d = add2(pack2(diff_of_products(t.x, v.x, t.y, v.y), sum_of_products(t.x, v.y, t.y, v.x)), dc);
+    const float2 n = unpack2(d);
+    z = unpack2(add2(pack2(z1.x, z1.y), d));
+    mag = sum_of_products(z.x, z.x, z.y, z.y);
+    dd = sum_of_products(n.x, n.x, n.y, n.y);
 }
 
 // round(hi + lo + d) for |lo| <= ulp(hi)/2: s = hi + d with its exact error, plus lo.
@@ -468,21 +465,86 @@ __global__ void __launch_bounds__(128, 8) k_perturb(const float2* __restrict__ o
     const float b2 = bailout * bailout;
     unsigned long long total = 0, rebases = 0;
     uint32_t pix = 0, m = 0, base = 0, stop = 0;
-    float dx = 0.0f, dy = 0.0f, dcx = 0.0f, dcy = 0.0f;
+    F2 d = 0, dc = 0;
     OrbitQuad at{};  // Z_m .. Z_(m+3)
     bool busy = false, live = true;
     for (;;) {
         // every lane of the warp reaches this point together
-        bool want = live && !busy;
-        uint32_t got = warp_fetch(work, want);
+        bool event = busy;  // or may have one: the chunk runs checked
+        if (busy && m + PERT_CHUNK < stop) {
+            event = false;
+            F2 e = d;
+            OrbitQuad q[PERT_CHUNK / 4 + 1];
+            q[0] = at;
+#pragma unroll
+            for (int k = 1; k <= PERT_CHUNK / 4; ++k) q[k] = load_quad(orbit + m + 4 * k);
+#pragma unroll
+            for (int j = 0; j < PERT_CHUNK; ++j) {
+                float2 z;
+                float mag, dd;
+                pert_step(q[j / 4].z[j % 4], q[(j + 1) / 4].z[(j + 1) % 4], dc, e, z, mag, dd);
+                event |= (mag > b2) | (mag < dd);
+            }
+            if (!event) {
+                d = e;
+                m += PERT_CHUNK;
+                at = q[PERT_CHUNK / 4];
+            }
+        }
+        // one vote a chunk while no lane has an event or waits for a pixel
+        if (!__any_sync(FULL_MASK, busy ? event : live)) continue;
+        if (event) {
+            bool done = false;
+            float mag = 0.0f;
+#pragma unroll 1
+            for (int j = 0; j < PERT_CHUNK; ++j) {
+                float2 z;
+                float dd;
+                const float2 z1 = orbit[m + 1];
+                pert_step(orbit[m], z1, dc, d, z, mag, dd);
+                ++m;
+                if (mag > b2) {
+                    done = true;
+                    break;
+                }
+                const bool small = mag < dd;
+                if (small || m >= stop) {
+                    if (base + m >= max_iter) {
+                        done = true;
+                        break;
+                    }
+                    if (small || m + 1 >= M) {
+                        const float2 lo = orbit_lo[m], v = unpack2(d);
+                        d = pack2(add3(z1.x, lo.x, v.x, z.x), add3(z1.y, lo.y, v.y, z.y));
+                        base += m;
+                        m = 0;
+                        stop = min(max_iter - base, M - 1);
+                        at = load_quad(orbit);
+                        ++rebases;
+                        break;
+                    }
+                }
+            }
+            if (done) {
+                const uint32_t n = base + m;
+                iters[pix] = n;
+                total += n;
+                float r = sqrtf(mag);
+                smooth[pix] = n < max_iter ? float(n) + 1.0f - logf(logf(fmaxf(r, 1.0001f))) / logf(2.0f) : float(n);
+                busy = false;
+            }
+        }
+        __syncwarp();
+        const bool want = live && !busy;
+        const uint32_t got = warp_fetch(work, want);
         if (want) {
             if (got < N) {
                 pix = got;
                 uint32_t px = pix % width, py = pix / width;
                 // offset from c_ref = centre hi: the centre's lo part plus the pixel's position
-                dcx = __fadd_rn(c_lo.x, (float(px) - float(width) * 0.5f + 0.5f) * pitch);
-                dcy = __fadd_rn(c_lo.y, (float(height) * 0.5f - float(py) - 0.5f) * pitch);
-                dx = dy = 0.0f;
+                dc = pack2(__fadd_rn(c_lo.x, (float(px) - float(width) * 0.5f + 0.5f) * pitch),
+                           __fadd_rn(c_lo.y, (float(height) * 0.5f - float(py) - 0.5f) * pitch));
+                d = pack2(0.0f, 0.0f);
                 m = base = 0;
                 stop = min(max_iter, M - 1);
                 at = load_quad(orbit);
@@ -492,72 +554,6 @@ __global__ void __launch_bounds__(128, 8) k_perturb(const float2* __restrict__ o
             }
         }
         if (!__any_sync(FULL_MASK, busy)) break;
-        bool event = busy;  // or may have one: the chunk runs checked
-        if (busy && m + PERT_CHUNK < stop) {
-            event = false;
-            float x = dx, y = dy;
-            OrbitQuad q[PERT_CHUNK / 4 + 1];
-            q[0] = at;
-#pragma unroll
-            for (int k = 1; k <= PERT_CHUNK / 4; ++k) q[k] = load_quad(orbit + m + 4 * k);
-#pragma unroll
-            for (int j = 0; j < PERT_CHUNK; ++j) {
-                float zx, zy, mag, dd;
-                pert_step(q[j / 4].z[j % 4], q[(j + 1) / 4].z[(j + 1) % 4], dcx, dcy, x, y, zx, zy, mag, dd);
-                event |= (mag > b2) | (mag < dd);
-            }
-            if (!event) {
-                dx = x;
-                dy = y;
-                m += PERT_CHUNK;
-                at = q[PERT_CHUNK / 4];
-            }
-        }
-        __syncwarp();
-        if (__any_sync(FULL_MASK, event)) {
-            if (event) {
-                bool done = false;
-                float mag = 0.0f;
-#pragma unroll 1
-                for (int j = 0; j < PERT_CHUNK; ++j) {
-                    float zx, zy, dd;
-                    const float2 z1 = orbit[m + 1];
-                    pert_step(orbit[m], z1, dcx, dcy, dx, dy, zx, zy, mag, dd);
-                    ++m;
-                    if (mag > b2) {
-                        done = true;
-                        break;
-                    }
-                    const bool small = mag < dd;
-                    if (small || m >= stop) {
-                        if (base + m >= max_iter) {
-                            done = true;
-                            break;
-                        }
-                        if (small || m + 1 >= M) {
-                            const float2 lo = orbit_lo[m];
-                            dx = add3(z1.x, lo.x, dx, zx);
-                            dy = add3(z1.y, lo.y, dy, zy);
-                            base += m;
-                            m = 0;
-                            stop = min(max_iter - base, M - 1);
-                            at = load_quad(orbit);
-                            ++rebases;
-                            break;
-                        }
-                    }
-                }
-                if (done) {
-                    const uint32_t n = base + m;
-                    iters[pix] = n;
-                    total += n;
-                    float r = sqrtf(mag);
-                    smooth[pix] = n < max_iter ? float(n) + 1.0f - logf(logf(fmaxf(r, 1.0001f))) / logf(2.0f) : float(n);
-                    busy = false;
-                }
-            }
-            __syncwarp();
-        }
     }
     warp_stat(&stats[SF_STAT_DE_ITERS], total);
     warp_stat(&stats[SF_STAT_STEPS], rebases);

@@ -19,10 +19,10 @@ enum { TL_IDLE = 0, TL_MARCH = 1, TL_CAND = 2, TL_NORMAL = 3, TL_DONE = 4, TL_IN
 #define SF_FORM_ANY 99u  // the generic interpreter
 
 // fp: the form's constants, P's own or those of the launch (TraceLaunch.fp).
-template <int FORM>
+template <int FORM, bool BATCH = false>
 __device__ __forceinline__ DeRaw de_form(const DeProgram& P, const FormParams& fp, float3 p) {
-    if constexpr (FORM == SF_FORM_BULB) return de_bulb(fp, p);
-    else if constexpr (FORM == SF_FORM_BOX) return de_box(fp, p);
+    if constexpr (FORM == SF_FORM_BULB) return de_bulb<BATCH>(fp, p);
+    else if constexpr (FORM == SF_FORM_BOX) return de_box<BATCH>(fp, p);
     else if constexpr (FORM == SF_FORM_MENGER) return de_menger(fp, p);
     else return de_generic(P, p, false);
 }
@@ -228,7 +228,7 @@ __device__ __forceinline__ void trace_group(const DeProgram& P, const DevScene& 
             const DeProgram& Pq = MULTI ? *Pl : P;
             const FormParams& fq = MULTI ? Pl->fp : tl.fp;
             if (OPTICS && FORM == SF_FORM_ANY && exact_state) s = de_form_exact<FORM>(Pq, fq, q);
-            else s = de_form<FORM>(Pq, fq, q);
+            else s = de_form<FORM, MULTI>(Pq, fq, q);
             n_eval++;
             n_iter += s.iter;
             if constexpr (FORM == SF_FORM_ANY) {
