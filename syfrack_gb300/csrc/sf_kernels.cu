@@ -623,6 +623,15 @@ cudaError_t sf_launch_primary(uint32_t form, const DeProgram* prog, const DevSce
     default: return sf_launch_primary_any(prog, scene, pl, st);
     }
 }
+cudaError_t sf_launch_paths(uint32_t form, const DeProgram* prog, const DevScene* scene, PathSoA soa, DispatchGeom g,
+                            FilmPlanes film, unsigned long long* stats, uint32_t* work, cudaStream_t st) {
+    switch (form) {
+    case SF_FORM_BULB: return sf_launch_paths_bulb(prog, scene, soa, g, film, stats, work, st);
+    case SF_FORM_BOX: return sf_launch_paths_box(prog, scene, soa, g, film, stats, work, st);
+    case SF_FORM_MENGER: return sf_launch_paths_menger(prog, scene, soa, g, film, stats, work, st);
+    default: return sf_launch_paths_any(prog, scene, soa, g, film, stats, work, st);
+    }
+}
 cudaError_t sf_launch_generate(const DevScene* scene, PathSoA soa, DispatchGeom g, uint32_t* counts, cudaStream_t st) {
     k_generate<<<(g.paths + 255) / 256, 256, g.light_smem, st>>>(scene, soa, g, counts);
     return cudaGetLastError();

@@ -241,6 +241,19 @@ cudaError_t sf_launch_preview(const DeProgram* prog, const DevScene* scene, uint
 cudaError_t sf_launch_film_clear(FilmPlanes film, cudaStream_t st);
 cudaError_t sf_launch_megakernel(const DeProgram* prog, const DevScene* scene, uint32_t rich, PathSoA soa, DispatchGeom g,
                                  FilmPlanes film, unsigned long long* stats, cudaStream_t st);
+// Whole paths on persistent lanes (sf_path_kernel.cuh), one instantiation per form: scenes
+// without rich surfaces and fog, at most SF_MAX_SHADOWS shadow segments a bounce. *work is
+// the dispatch's path counter and must be 0 when it starts.
+cudaError_t sf_launch_paths(uint32_t form, const DeProgram* prog, const DevScene* scene, PathSoA soa, DispatchGeom g,
+                            FilmPlanes film, unsigned long long* stats, uint32_t* work, cudaStream_t st);
+cudaError_t sf_launch_paths_bulb(const DeProgram*, const DevScene*, PathSoA, DispatchGeom, FilmPlanes,
+                                 unsigned long long*, uint32_t*, cudaStream_t);
+cudaError_t sf_launch_paths_box(const DeProgram*, const DevScene*, PathSoA, DispatchGeom, FilmPlanes,
+                                unsigned long long*, uint32_t*, cudaStream_t);
+cudaError_t sf_launch_paths_menger(const DeProgram*, const DevScene*, PathSoA, DispatchGeom, FilmPlanes,
+                                   unsigned long long*, uint32_t*, cudaStream_t);
+cudaError_t sf_launch_paths_any(const DeProgram*, const DevScene*, PathSoA, DispatchGeom, FilmPlanes,
+                                unsigned long long*, uint32_t*, cudaStream_t);
 cudaError_t sf_launch_planar(const PlanarDev* f, const float* x, const float* y, size_t n, float* dist, float* traps,
                              uint32_t* iters, cudaStream_t st);
 // with_traps = 0 writes only dist, traps[0 .. n) (smooth time) and iters. *work is
