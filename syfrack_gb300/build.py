@@ -16,9 +16,10 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libsyfrack_gpu.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-UNITS = ["sf_kernels.cu", "sf_escape.cu", "sf_trace_box.cu", "sf_trace_bulb.cu", "sf_trace_menger.cu", "sf_trace_any.cu",
+UNITS = ["sf_mega.cu", "sf_mega_rich.cu", "sf_mega_textured.cu", "sf_batch.cu", "sf_kernels.cu", "sf_escape.cu",
+         "sf_trace_box.cu", "sf_trace_bulb.cu", "sf_trace_menger.cu", "sf_trace_any.cu",
          "sf_paths_box.cu", "sf_paths_bulb.cu", "sf_paths_menger.cu", "sf_paths_any.cu",
-         "sf_batch.cu", "sf_batch_generic.cu", "sf_noalloc.cu", "sf_preview.cu", "sf_host.cpp", "sf_batch_host.cpp",
+         "sf_batch_generic.cu", "sf_noalloc.cu", "sf_preview.cu", "sf_host.cpp", "sf_batch_host.cpp",
          "sf_serve.cpp", "sf_export.cpp", "sf_preview.cpp", "sf_environment.cpp"]
 
 

@@ -241,6 +241,10 @@ cudaError_t sf_launch_preview(const DeProgram* prog, const DevScene* scene, uint
 cudaError_t sf_launch_film_clear(FilmPlanes film, cudaStream_t st);
 cudaError_t sf_launch_megakernel(const DeProgram* prog, const DevScene* scene, uint32_t rich, PathSoA soa, DispatchGeom g,
                                  FilmPlanes film, unsigned long long* stats, cudaStream_t st);
+cudaError_t sf_launch_megakernel_rich(const DeProgram*, const DevScene*, PathSoA, DispatchGeom, FilmPlanes,
+                                      unsigned long long*, cudaStream_t);
+cudaError_t sf_launch_megakernel_textured(const DeProgram*, const DevScene*, PathSoA, DispatchGeom, FilmPlanes,
+                                          unsigned long long*, cudaStream_t);
 // Whole paths on persistent lanes (sf_path_kernel.cuh), one instantiation per form: scenes
 // without rich surfaces and fog, at most SF_MAX_SHADOWS shadow segments a bounce. *work is
 // the dispatch's path counter and must be 0 when it starts.
