@@ -348,7 +348,7 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 // 2 clamp(x, -l, l) - x of the box fold, bit for bit but for the sign of a zero, in two
 // instructions for three: with t = 2 l - |x| it is the smaller of |x| and |t|, with the
 // sign of x times that of t. (|x| <= l: t rounds to no less than |x|. Past l, t is the
-// fold of |x|, rounded once as the fused form is, and |t| <= |x|.) 0 <= l, 2 l finite.
+// fold of |x|, rounded once as the fused form is, and |t| <= |x|.) 0 <= l <= 1e38.
 __device__ __forceinline__ float box_fold(float x, float l2) {
     float q;
     asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(q) : "f"(x), "f"(l2 - fabsf(x)));
@@ -425,10 +425,40 @@ __device__ __forceinline__ DeRaw de_box_c(const FormParams& f, float3 p) {
     if (BATCH) return de_box_t<NORM_MIN0, CLAMPED, 0>(f, p);
     return f.scale < 0.0f ? de_box_t<NORM_MIN0, CLAMPED, -1>(f, p) : de_box_t<NORM_MIN0, CLAMPED, 1>(f, p);
 }
+// Limits that box_fold() does not take (negative, above 1e38, not a number): the plain
+// clamp, every option read as it runs. Rare, so one small loop; the form stays the
+// graph's whatever its values.
+__device__ __forceinline__ DeRaw de_box_any_limit(const FormParams& f, float3 p) {
+    DeRaw s = raw_empty();
+    float dr = 1.0f;
+    const float3 c = p;
+    const float l = f.limit;
+    const bool sq = f.trap_squared != 0;
+    auto fold = [&](float x) { return fmaf(fminf(fmaxf(-x, -l), l), -2.0f, -x); };
+    uint32_t i = 0;
+#pragma unroll 1
+    for (; i < f.iterations; ++i) {
+        if (dot3(p, p) > f.bailout_t) break;
+        const float3 q = mk3(fold(p.x), fold(p.y), fold(p.z));
+        const float r2 = dot3(q, q);
+        trap_update(s, f.trap_slot, f.trap_mode, sq ? r2 : trap_measure(f.trap_measure, q));
+        const float qk = fmaxf(f.fixed_radius2 * rcp_approx(r2), 1.0f);
+        const float k = f.fold_clamped ? fminf(f.fold_k_min, qk) : (r2 < f.min_radius2 ? f.fold_k_min : qk);
+        const float ks = k * f.scale;
+        p = mk3(fmaf(q.x, ks, c.x), fmaf(q.y, ks, c.y), fmaf(q.z, ks, c.z));
+        dr = fmaf(dr, k * fabsf(f.scale), 1.0f);
+    }
+    s.iter = i;
+    s.d = (sqrt_fast(dot3(p, p)) - f.fence[0]) * rcp_approx(fabsf(dr));
+    s.material = f.material;
+    if (sq && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM) s.t0 = sqrt_fast(s.t0);
+    else if (sq) trap_sqrt(s, f.trap_slot);
+    return s;
+}
 template <bool BATCH = false>
 __device__ __forceinline__ DeRaw de_box(const FormParams& f, float3 p) {
-    if (f.trap_squared && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM)
-        return f.fold_clamped ? de_box_c<true, true, BATCH>(f, p) : de_box_c<true, false, BATCH>(f, p);
+    if (f.box_plain) return f.fold_clamped ? de_box_c<true, true, BATCH>(f, p) : de_box_c<true, false, BATCH>(f, p);
+    if (!f.box_limit) return de_box_any_limit(f, p);
     return f.fold_clamped ? de_box_c<false, true, BATCH>(f, p) : de_box_c<false, false, BATCH>(f, p);
 }
 

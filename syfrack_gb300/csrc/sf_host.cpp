@@ -652,10 +652,11 @@ void detect_form(const HostGraph& g, DeProgram& P) {
         f.power_int = (pw >= 1.f && pw <= 16.f && pw == std::floor(pw)) ? uint32_t(pw) : 0u;
         P.form = SF_FORM_BULB;
     } else if (fence->kind == SF_NODE_NORM_FENCE &&
-               kinds({SF_NODE_BOX_FOLD, SF_NODE_TRAP, SF_NODE_SPHERE_FOLD, SF_NODE_SCALE, SF_NODE_ADD_ORIGIN}) &&
-               body[0]->f[0] >= 0.0f && body[0]->f[0] <= 1e38f) {  // the limits box_fold() takes
+               kinds({SF_NODE_BOX_FOLD, SF_NODE_TRAP, SF_NODE_SPHERE_FOLD, SF_NODE_SCALE, SF_NODE_ADD_ORIGIN})) {
         f.limit = body[0]->f[0];
         set_trap(body[1]);
+        f.box_limit = f.limit >= 0.0f && f.limit <= 1e38f;  // what box_fold() takes
+        f.box_plain = f.box_limit && f.trap_squared && f.trap_slot == 0 && f.trap_mode == SF_TRAP_MINIMUM;
         float mr = body[2]->f[0], fr = body[2]->f[1];
         f.min_radius2 = mr * mr;
         f.fixed_radius2 = fr * fr;

@@ -20,7 +20,8 @@
 #define SF_MAX_INST_DEPTH 3  // nested Instances levels (MAX_DEPTH, graph/mod.rs:41)
 #define SF_MAX_UNION_LEAVES 32  // leaves of the exact union branch-and-bound
 
-// Opcodes of the generic interpreter. Point and fence operations use the node
+// Opcodes of the generic interpreter (some operations' unused f hold constants prepared on
+// the device when the program is uploaded: prepare_op in sf_de.cuh). Point and fence operations use the node
 // kind (enum sf_node_kind) as their code; control codes start at 100.
 enum {
     SF_OP_BEGIN = 100,      // point state := input point
@@ -36,13 +37,16 @@ enum {
     // port-0 point chain and computes bound = box(point, f0..2); in fast mode, when
     // bound > f3 (margin), it pushes {bound, no traps, 0 iterations, material 0,
     // flags 1} and jumps past the detail branch to b; otherwise it pushes the bound
-    // and the detail branch follows, closed by BOUND_END.
+    // and the detail branch follows, closed by BOUND_END. a = the unions pending on the
+    // distance stack whose first operand it may lose to (0 = none): a bound that cannot
+    // beat it leaves the branch out in exact mode too.
     SF_OP_BOUND_FAST = 109,
     SF_OP_BOUND_END = 110,  // detail.d = max(bound, detail.d); the detail's payload and flags stay
     // Instances (graph_wgsl.rs:744-790): a = placement count, b = index of INST_END,
     // c = offset of the node's block in inst_data (12 floats of inverse affine rows per
     // placement, then 8 floats per hierarchy node: centre, half, escape, placement or -1),
-    // f0..2 = half, f3 = margin, f4 = 1 when the copies may be skipped (fast). The ops
+    // f0..2 = half, f3 = margin, f4 = 1 when the copies may be skipped (fast), f5 =
+    // the pending unions, as BOUND_FAST's a. The ops
     // between INST_BEGIN and INST_END evaluate the template at a copy's local point;
     // they may hold further Instances, nested up to SF_MAX_INST_DEPTH levels.
     SF_OP_INST_BEGIN = 111,
@@ -65,6 +69,8 @@ struct FormParams {
     float power;         // Bulb
     uint32_t power_int;  // Bulb: 0 = trigonometric path, else the integer exponent 1..16
     float limit;         // Box: fold limit
+    uint32_t box_limit;  // Box: 0 <= limit <= 1e38, the two-instruction fold applies
+    uint32_t box_plain;  // Box: that, and the bundled trap (slot 0, Norm, Minimum)
     float min_radius2, fixed_radius2, fold_k_min;  // Box: mr^2, fr^2, fr^2/mr^2
     uint32_t fold_clamped;  // Box: fr >= mr, so the fold factor is min(fr^2/mr^2, max(fr^2/r^2, 1))
     float scale;         // Box: Scale factor; Menger: fold scale

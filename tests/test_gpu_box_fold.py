@@ -1,7 +1,8 @@
 """The Mandelbox form's two-instruction fold and its loop of iteration pairs: limits of
 zero, inside and past the points, and the largest it takes, with odd and even iteration
-counts; limits outside 0..1e38 run on the generic interpreter. All follow the f32 oracle
-(the rule and the few-ulp quantile of the form tests)."""
+counts; a limit past 1e38 takes the plain loop. All follow the f32 oracle (the rule and the
+few-ulp quantile of the form tests). A negative limit, where clamp(-x, -l, l) is l, folds x
+to -2 l - x on this form; a value edit between the two kinds reaches a batch that exists."""
 import numpy as np
 import pytest
 
@@ -12,13 +13,12 @@ from test_gpu_de import gpu_de_rule
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("limit,form", [(0.0, "box"), (0.35, "box"), (1.0, "box"), (2.5, "box"), (1e38, "box"),
-                                        (-0.5, "generic"), (2e38, "generic")])
+@pytest.mark.parametrize("limit", [0.0, 0.35, 1.0, 2.5, 1e38, 2e38])
 @pytest.mark.parametrize("iterations", [1, 2, 3, 4])
-def test_limits_and_iteration_pairs(renderer, oracle_mod, limit, form, iterations):
+def test_limits_and_iteration_pairs(renderer, oracle_mod, limit, iterations):
     g = Graph.bundled("mandelbox", limit=limit, iterations=iterations, scale=-1.5, bailout=1000.0)
     cg = renderer.compile(g)
-    assert cg.info()["form"] == form
+    assert cg.info()["form"] == "box"
     pts = lcg_points(4096, 4.0, 21 + iterations)
     pts[:8] = [(x, y, z) for x in (0.35, -0.7) for y in (1.0, -2.0) for z in (2.5, 0.0)]  # at l and 2 l
     gpu = cg.probe(pts)
@@ -27,3 +27,54 @@ def test_limits_and_iteration_pairs(renderer, oracle_mod, limit, form, iteration
     rel = np.abs(gpu["distance"] - ref["distance"]) / np.maximum(np.abs(ref["distance"]), 1.0)
     assert np.quantile(rel, 0.99) < 1e-5
     assert (gpu["iterations"] == ref["iterations"]).mean() >= 0.995
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 3])
+def test_negative_limit(renderer, iterations):
+    limit, scale = -0.5, -1.5
+    g = Graph.bundled("mandelbox", limit=limit, iterations=iterations, scale=scale, bailout=1000.0)
+    pts = lcg_points(4096, 2.0, 33)
+    gpu = renderer.compile(g).probe(pts)
+    p = c = pts.astype(np.float64)
+    dr = np.ones(len(pts))
+    for _ in range(iterations):
+        q = -2.0 * limit - p
+        k = np.minimum(4.0, np.maximum(1.0 / (q * q).sum(1), 1.0))  # radii 0.5 and 1
+        p, dr = q * (k * scale)[:, None] + c, dr * k * abs(scale) + 1.0
+    fence = [n for n in g.nodes if n.kind.name == "NormFence"][0].kind.fields["inset"]
+    ref = (np.linalg.norm(p, axis=1) - fence) / dr
+    rel = np.abs(gpu["distance"] - ref) / np.maximum(np.abs(ref), 1.0)
+    assert np.quantile(rel, 0.99) < 1e-5
+    assert np.all(gpu["iterations"] == iterations)
+
+
+def test_value_edit_across_the_limits(renderer):
+    """sf_graph_update from a limit of 1 to -0.5 and back: the batch made before renders as
+    one made after."""
+    from syfrack_gb300 import Batch, workloads
+    from syfrack_gb300.scene import RenderConfig
+
+    cfg = RenderConfig(48, 32, 2, max_bounces=2, max_steps=128, pixel_tolerance=1.0, tile_size=48,
+                       samples_per_dispatch=2, integrator="wavefront")
+
+    def film(scene, edit=None):
+        b = Batch(renderer, [(scene, cfg)])
+        if edit is not None:
+            edit(b)
+        b.run(1, use_graph=False)
+        assert b.sync() == 0
+        out = b.readback(0)
+        b.close()
+        return out
+
+    scene = workloads.mandelbox_scene()
+    other = workloads.mandelbox_scene()
+    for n in other.graph.nodes:
+        if n.kind.name == "BoxFold":
+            n.kind.fields["limit"] = -0.5
+    want = film(other)
+    cg = renderer.compile(scene.graph)
+    got = film(scene, lambda b: cg.update(other.graph))
+    cg.update(scene.graph)
+    np.testing.assert_array_equal(got.accum, want.accum)
+    np.testing.assert_array_equal(got.depth, want.depth)
