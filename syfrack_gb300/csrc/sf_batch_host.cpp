@@ -29,7 +29,7 @@ namespace sfh {
 
 // Carves an arena for `capacity` paths and `max_jobs` jobs out of one allocation.
 sf_status arena_alloc(sf_context* c, WaveArena& a, uint32_t capacity, uint32_t max_jobs, uint32_t rounds,
-                      uint32_t shadow_slots, size_t extra_bytes, size_t* extra_offset) {
+                      uint32_t shadow_slots, uint32_t groups, size_t extra_bytes, size_t* extra_offset) {
     const size_t N = capacity;
     const uint32_t K = std::max<uint32_t>(shadow_slots, 1);
     size_t off = 0;
@@ -37,7 +37,8 @@ sf_status arena_alloc(sf_context* c, WaveArena& a, uint32_t capacity, uint32_t m
     size_t o_jobs = take(size_t(max_jobs) * sizeof(BatchJob));
     size_t o_Ls = take(N * 16), o_soa = take(wave_soa_bytes(N, K)), o_lists = take(wave_lists_bytes(N, K));
     size_t o_march = take(wave_march_bytes(N, K)), o_resume = take(wave_resume_bytes(N, K));
-    size_t o_counts = take(wave_counts_bytes(rounds)), o_qcounts = take(wave_launch_counts_bytes(rounds));
+    size_t o_counts = take(wave_counts_bytes(rounds, groups));
+    size_t o_qcounts = take(wave_launch_counts_bytes(rounds, groups));
     size_t o_status = take(16);
     size_t o_extra = take(extra_bytes);
     sf_status st = ctx_alloc(c, off, &a.mem);
@@ -48,6 +49,7 @@ sf_status arena_alloc(sf_context* c, WaveArena& a, uint32_t capacity, uint32_t m
     a.capacity = capacity;
     a.max_jobs = max_jobs;
     a.rounds = rounds;
+    a.groups = groups;
     wave_bind(a.soa, base + o_soa, base + o_march, capacity, K);
     a.soa.Ls = reinterpret_cast<float4*>(base + o_Ls);
     a.lists = reinterpret_cast<uint32_t*>(base + o_lists);
@@ -93,8 +95,8 @@ sf_status wave_record_pass(sf_context* c, const WaveArena& a, cudaStream_t st, b
     const size_t N = a.capacity;
     const uint32_t R = a.rounds;
     const uint32_t Q = a.quantum ? std::min<uint32_t>((a.max_steps + a.quantum - 1) / a.quantum + 1, 64) : 1;
-    CU(cudaMemsetAsync(a.counts, 0, wave_counts_bytes(R), st));
-    CU(cudaMemsetAsync(a.qcounts, 0, wave_launch_counts_bytes(R), st));
+    CU(cudaMemsetAsync(a.counts, 0, wave_counts_bytes(R, a.groups), st));
+    CU(cudaMemsetAsync(a.qcounts, 0, wave_launch_counts_bytes(R, a.groups), st));
     {
         LaunchTimer t(c, false, timed, st);
         CU(sf_launch_generate_batch(a.bt, a.soa, a.counts, st));
@@ -103,12 +105,12 @@ sf_status wave_record_pass(sf_context* c, const WaveArena& a, cudaStream_t st, b
     const uint32_t K = a.soa.shadow_slots;
     for (uint32_t r = 0; r < R; ++r) {
         RoundQueues q;
-        wave_round_queues(q, a.lists, N, K, r, a.counts);
+        wave_round_queues(q, a.lists, N, K, r, a.counts, a.groups);
         for (uint32_t j = 0; j < Q; ++j) {
             TraceLaunch tl{};
             tl.q = q;
-            tl.counts = wave_launch_counts(a.qcounts, r, j);
-            tl.last_counts = j == 0 ? nullptr : wave_launch_counts(a.qcounts, r, j - 1);
+            tl.counts = wave_launch_counts(a.qcounts, r, j, a.groups);
+            tl.last_counts = j == 0 ? nullptr : wave_launch_counts(a.qcounts, r, j - 1, a.groups);
             tl.resume = j == 0 ? nullptr : wave_resume(a.resume, N, K, j - 1);
             tl.next_resume = wave_resume(a.resume, N, K, j);
             tl.quantum = j + 1 == Q ? 0u : a.quantum;
@@ -197,7 +199,11 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
     // details, textures and optics keep the footprint and medium row
     const size_t pv_bytes = any_fog ? size_t(paths) * 16 : 0;
     const size_t ex_bytes = rich ? size_t(paths) * 16 : 0;
-    sf_status st = arena_alloc(c, b->a, uint32_t(paths), n, rounds, K,
+    std::vector<const sf_graph*> graphs;
+    for (uint32_t i = 0; i < n; ++i) graphs.push_back(jobs[i].graph);
+    const std::vector<uint32_t> keys = group_keys(graphs);
+    const uint32_t groups = uint32_t(std::set<uint32_t>(keys.begin(), keys.end()).size());
+    sf_status st = arena_alloc(c, b->a, uint32_t(paths), n, rounds, K, groups,
                                scene_bytes + pv_bytes + ex_bytes + film_bytes, &extra);
     if (st != SF_OK) { delete b; return st; }
     b->a.max_steps = max_steps;
@@ -219,9 +225,6 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
     uint32_t pbeg = 0, xbeg = 0;
     std::vector<uint32_t> order(n);
     for (uint32_t i = 0; i < n; ++i) order[i] = i;
-    std::vector<const sf_graph*> graphs;
-    for (uint32_t i = 0; i < n; ++i) graphs.push_back(jobs[i].graph);
-    const std::vector<uint32_t> keys = group_keys(graphs);
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return keys[x] < keys[y]; });
     uint32_t last_key = 0;
     b->slot.resize(n);

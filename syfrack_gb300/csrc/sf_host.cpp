@@ -1679,8 +1679,8 @@ sf_status session_alloc(sf_session* s) {
         o_march = take(wave_march_bytes(N, K));
         o_resume = take(wave_resume_bytes(N, K));
     }
-    size_t o_counts = take(wave_counts_bytes(R));
-    size_t o_qcounts = take(wave_launch_counts_bytes(R));
+    size_t o_counts = take(wave_counts_bytes(R, 1));
+    size_t o_qcounts = take(wave_launch_counts_bytes(R, 1));
     size_t o_status = take(16);
     s->mem_bytes = off;
     sf_status st = ctx_alloc(c, off, &s->mem);
@@ -1819,8 +1819,8 @@ extern "C" sf_status sf_session_dispatch(sf_session* s, sf_tile tile, uint32_t s
     const size_t N = s->capacity;
     // launches per round: the first, then one per step quantum a segment may still need
     const uint32_t Q = s->quantum ? std::min<uint32_t>((s->cfg.max_steps + s->quantum - 1) / s->quantum + 1, 64) : 1;
-    CU(cudaMemsetAsync(s->counts, 0, wave_counts_bytes(R), st));
-    CU(cudaMemsetAsync(s->qcounts, 0, wave_launch_counts_bytes(R), st));
+    CU(cudaMemsetAsync(s->counts, 0, wave_counts_bytes(R, 1), st));
+    CU(cudaMemsetAsync(s->qcounts, 0, wave_launch_counts_bytes(R, 1), st));
     {
         LaunchTimer t(c, false);
         CU(sf_launch_generate(s->d_scene, s->soa, g, s->counts, st));
@@ -1831,12 +1831,12 @@ extern "C" sf_status sf_session_dispatch(sf_session* s, sf_tile tile, uint32_t s
     const uint32_t K = s->shadow_slots;
     for (uint32_t r = 0; r < R; ++r) {
         RoundQueues q;
-        wave_round_queues(q, s->lists, N, K, r, s->counts);
+        wave_round_queues(q, s->lists, N, K, r, s->counts, 1);
         for (uint32_t j = 0; j < Q; ++j) {
             TraceLaunch tl{};
             tl.q = q;
-            tl.counts = wave_launch_counts(s->qcounts, r, j);
-            tl.last_counts = j == 0 ? nullptr : wave_launch_counts(s->qcounts, r, j - 1);
+            tl.counts = wave_launch_counts(s->qcounts, r, j, 1);
+            tl.last_counts = j == 0 ? nullptr : wave_launch_counts(s->qcounts, r, j - 1, 1);
             tl.resume = j == 0 ? nullptr : wave_resume(s->resume, N, K, j - 1);
             tl.next_resume = wave_resume(s->resume, N, K, j);
             tl.quantum = j + 1 == Q ? 0u : s->quantum;  // the last launch runs segments to completion

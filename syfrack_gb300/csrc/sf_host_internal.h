@@ -215,25 +215,28 @@ inline void wave_bind(PathSoA& soa, void* soa_mem, void* march_mem, uint32_t N, 
     soa.capacity = N;
     soa.shadow_slots = K;
 }
-inline void wave_round_queues(RoundQueues& q, uint32_t* lists, size_t N, uint32_t K, uint32_t r, uint32_t* counts) {
+inline void wave_round_queues(RoundQueues& q, uint32_t* lists, size_t N, uint32_t K, uint32_t r, uint32_t* counts,
+                              uint32_t groups) {
     const size_t stride = (2 + size_t(K)) * N;
     uint32_t* cur = lists + (r & 1) * stride;
     uint32_t* nxt = lists + ((r & 1) ^ 1) * stride;
     q.active = r == 0 ? nullptr : cur;
     q.cont = r == 0 ? nullptr : cur + N;
     q.shadow = cur + 2 * N;
-    q.counts = counts + SF_ROUND_COUNTS * r;
+    q.counts = counts + size_t(SF_ROUND_COUNTS(groups)) * r;
     q.next_active = nxt;
     q.next_cont = nxt + N;
     q.next_shadow = nxt + 2 * N;
-    q.next_counts = counts + SF_ROUND_COUNTS * (r + 1);
+    q.next_counts = counts + size_t(SF_ROUND_COUNTS(groups)) * (r + 1);
 }
 // Counters of R rounds (and the one after) and of their launches, at most 64 a round.
-inline size_t wave_counts_bytes(uint32_t R) { return size_t(R + 1) * SF_ROUND_COUNTS * 4; }
-inline size_t wave_launch_counts_bytes(uint32_t R) { return size_t(R) * 64 * SF_LAUNCH_COUNTS * 4; }
+inline size_t wave_counts_bytes(uint32_t R, uint32_t groups) { return size_t(R + 1) * SF_ROUND_COUNTS(groups) * 4; }
+inline size_t wave_launch_counts_bytes(uint32_t R, uint32_t groups) {
+    return size_t(R) * 64 * SF_LAUNCH_COUNTS(groups) * 4;
+}
 // Launch j of round r: its counters and resume lists.
-inline uint32_t* wave_launch_counts(uint32_t* qcounts, uint32_t r, uint32_t j) {
-    return qcounts + (size_t(r) * 64 + j) * SF_LAUNCH_COUNTS;
+inline uint32_t* wave_launch_counts(uint32_t* qcounts, uint32_t r, uint32_t j, uint32_t groups) {
+    return qcounts + (size_t(r) * 64 + j) * SF_LAUNCH_COUNTS(groups);
 }
 inline uint32_t* wave_resume(uint32_t* resume, size_t N, uint32_t K, uint32_t parity) {
     return resume + size_t(parity & 1) * (1 + size_t(K)) * N;
@@ -244,6 +247,7 @@ struct WaveArena {
     BatchTable bt{};
     PathSoA soa{};
     uint32_t capacity = 0, rounds = 0, max_steps = 0, max_jobs = 0;
+    uint32_t groups = 0;  // what the counters hold: at least bt.groups
     uint32_t* lists = nullptr;
     uint32_t* resume = nullptr;
     uint32_t* counts = nullptr;
@@ -266,7 +270,7 @@ std::vector<uint32_t> group_keys(const std::vector<const sf_graph*>& graphs);
 // path_begin if the job opens it.
 uint32_t group_of(BatchTable& bt, uint32_t& last_key, uint32_t key, uint32_t form, uint32_t path_begin);
 sf_status arena_alloc(sf_context* c, WaveArena& a, uint32_t capacity, uint32_t max_jobs, uint32_t rounds,
-                      uint32_t shadow_slots, size_t extra_bytes, size_t* extra_offset);
+                      uint32_t shadow_slots, uint32_t groups, size_t extra_bytes, size_t* extra_offset);
 sf_status wave_record_pass(sf_context* c, const WaveArena& a, cudaStream_t st, bool timed);
 
 }  // namespace sfh

@@ -57,9 +57,9 @@ struct PathSoA {
 // Counters of a round: active paths, then per group of jobs its continuation and its
 // shadow segments (a session is one group, a batch one per form and variant of it).
 #define SF_MAX_GROUPS 8
-#define SF_ROUND_COUNTS (1 + 2 * SF_MAX_GROUPS)
+#define SF_ROUND_COUNTS(groups) (1 + 2 * (groups))
 // Counters of one trace launch: per group {work counter, resumed segments}.
-#define SF_LAUNCH_COUNTS (2 * SF_MAX_GROUPS)
+#define SF_LAUNCH_COUNTS(groups) (2 * (groups))
 
 // Queues of one round: active paths, continuation rays, shadow rays (ids), with their
 // SF_ROUND_COUNTS counters; next round's lists are written by shade. A group whose

@@ -600,7 +600,7 @@ extern "C" sf_status sf_server_create(sf_context* c, const sf_server_config* cfg
         if (e != cudaSuccess) return bail(cuda_fail(e, "server slot"));
         size_t ex_off = 0;
         sf_status st = arena_alloc(c, sl.arena, k.path_capacity, k.max_jobs, max_rounds, kServeShadowSlots,
-                                   size_t(k.path_capacity) * 16, &ex_off);
+                                   SF_MAX_GROUPS, size_t(k.path_capacity) * 16, &ex_off);
         if (st != SF_OK) return bail(st);
         sl.arena.soa.ex = reinterpret_cast<float4*>(static_cast<char*>(sl.arena.mem) + ex_off);
         sl.arena.min_blocks = k.min_blocks;
