@@ -1419,6 +1419,9 @@ extern "C" sf_status sf_graph_validate(const sf_graph_desc* d, sf_graph_info* ou
     if (s == SF_OK && out) *out = info;
     return s;
 }
+// The specialised forms never run their ops, so those need no preparation (a launch and a
+// wait for it, 20 us of a compile).
+static bool interpreted(const DeProgram& P) { return P.form == SF_FORM_GENERIC && P.n_ops != 0; }
 extern "C" sf_status sf_graph_compile(sf_context* c, const sf_graph_desc* d, sf_graph** out) {
     if (!c || !out) return fail(SF_ERR_INVALID, "null argument");
     *out = nullptr;
@@ -1448,7 +1451,7 @@ extern "C" sf_status sf_graph_compile(sf_context* c, const sf_graph_desc* d, sf_
     if (g->d_inst) e = cudaMemcpyAsync(g->d_inst, inst.data(), g->inst_bytes, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(g->d_prog, &g->prog, sizeof(DeProgram), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess && g->prog.n_ops) e = sf_launch_prepare_program(g->d_prog, c->stream);
+    if (e == cudaSuccess && interpreted(g->prog)) e = sf_launch_prepare_program(g->d_prog, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         ctx_free(c, g->d_prog, sizeof(DeProgram));
@@ -1480,7 +1483,7 @@ extern "C" sf_status sf_graph_update(sf_graph* g, const sf_graph_desc* d) {
     CU(cudaDeviceSynchronize());  // no launch on any stream (previews, server slots) may read what is replaced
     if (g->d_inst) CU(cudaMemcpyAsync(g->d_inst, inst.data(), g->inst_bytes, cudaMemcpyHostToDevice, g->ctx->stream));
     CU(cudaMemcpyAsync(g->d_prog, &P, sizeof P, cudaMemcpyHostToDevice, g->ctx->stream));
-    if (P.n_ops) CU(sf_launch_prepare_program(g->d_prog, g->ctx->stream));
+    if (interpreted(P)) CU(sf_launch_prepare_program(g->d_prog, g->ctx->stream));
     CU(cudaStreamSynchronize(g->ctx->stream));
     g->host = h;
     g->prog = P;
