@@ -654,7 +654,9 @@ typedef struct sf_server_config {
     uint32_t path_capacity;     /* paths per 3D batch (a request needs w*h*samples)   */
     uint32_t max_jobs;          /* requests per batch, 1..1024                        */
     uint32_t max_tile_pixels;   /* 2D pixels per batch                                */
-    uint32_t min_blocks, quantum, regen; /* trace launch shape (sf_batch_set_launch)  */
+    uint32_t min_blocks, quantum, regen; /* trace launch shape (sf_batch_set_launch);
+                                          * a batch of 2M paths or fewer is not split by
+                                          * the quantum                               */
     uint32_t pad;
 } sf_server_config;
 typedef struct sf_request {

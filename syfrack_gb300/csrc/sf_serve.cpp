@@ -166,6 +166,11 @@ struct ServeReq {
 };
 
 constexpr uint32_t kServeMaxSlots = 8;
+// A batch of up to this many paths (about 18 for each lane of 3 blocks an SM) marches its
+// segments in one launch a round whatever the step quantum: the launches that only carry
+// on at a quantum cost it more than the shorter tails give. One 480x270 preview 2.25 ms
+// with quanta of 128 steps and 1.91 without, 8 previews and 4 refinements 16.7 and 15.3.
+constexpr uint32_t kServeUnsplitPaths = 1u << 21;
 constexpr uint32_t kServeShadowSlots = 3;  // shadow segments per bounce the slot arenas hold
 constexpr uint32_t kServeMaxTiles = 64;  // 2D tiles per batch
 // A tile's device block starts with PlanarDev (0), CanvasDev (256) and its pixel
@@ -366,6 +371,8 @@ sf_status launch_wave(sf_server* s, ServeSlot& sl) {
     // rounds vary per batch; the arena's queue counters are sized for its largest
     WaveArena pass = a;
     pass.rounds = rounds;
+    pass.groups = a.bt.groups;  // and its groups
+    if (paths <= kServeUnsplitPaths) pass.quantum = 0;
     // scenes with finish details, a texture or optics: the feature-built kernels and the
     // footprint and medium rows (kept by the slot, unused by plain batches)
     pass.rich = rich;
