@@ -345,8 +345,8 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     return r;
 }
 
-// 2 clamp(x, -l, l) - x of the box fold, bit for bit but for the sign of a zero, in two
-// instructions for three: with t = 2 l - |x| it is the smaller of |x| and |t|, with the
+// 2 clamp(x, -l, l) - x of the box fold, bit for bit but for the sign of a zero (the
+// clamped form's zeros are +0, see the trap in de_box_t), in two instructions for three: with t = 2 l - |x| it is the smaller of |x| and |t|, with the
 // sign of x times that of t. (|x| <= l: t rounds to no less than |x|. Past l, t is the
 // fold of |x|, rounded once as the fused form is, and |t| <= |x|.) 0 <= l <= 1e38.
 __device__ __forceinline__ float box_fold(float x, float l2) {
@@ -386,7 +386,8 @@ __device__ __forceinline__ DeRaw de_box_t(const FormParams& f, float3 p) {
         const float3 q = mk3(box_fold(p.x, l2), box_fold(p.y, l2), box_fold(p.z, l2));
         const float r2 = dot3(q, q);
         if (!NORM_MIN0) {
-            float v = sq ? r2 : trap_measure(f.trap_measure, q);
+            // an angle sees the sign of a zero: + 0 makes it the clamped form's (a folded zero is +0)
+            float v = sq ? r2 : trap_measure(f.trap_measure, mk3(q.x + 0.0f, q.y + 0.0f, q.z + 0.0f));
             trap_update(s, f.trap_slot, f.trap_mode, v);
         }
         const float qk = fr2 * rcp_approx(r2);

@@ -78,3 +78,20 @@ def test_value_edit_across_the_limits(renderer):
     cg.update(scene.graph)
     np.testing.assert_array_equal(got.accum, want.accum)
     np.testing.assert_array_equal(got.depth, want.depth)
+
+
+@pytest.mark.parametrize("measure", ["AngleXY", "AngleXZ", "AngleYZ"])
+@pytest.mark.parametrize("limit", [0.5, 1.0])
+def test_angles_of_folded_lattice_points(renderer, oracle_mod, measure, limit):
+    """Components that fold to zero (0, -0 and both ends 2 l, -2 l) fold to +0: an angle on
+    the negative axis is pi, not -pi. One iteration, so the folds are exact and the angle
+    is within 3 ulp of pi (7e-7) over 2 pi, plus the rounding of the sum with a half."""
+    g = Graph.bundled("mandelbox", limit=limit, iterations=1, scale=-1.5, bailout=1000.0, trap_scale=1.0)
+    for n in g.nodes:
+        if n.kind.name == "Trap":
+            n.kind.fields["measure"] = measure
+    axis = np.array([-4.0, -2.0, -1.4, -1.0, -0.6, -0.0, 0.0, 0.6, 1.0, 1.4, 2.0, 4.0], np.float32) * np.float32(limit)
+    pts = np.stack(np.meshgrid(axis, axis, axis, indexing="ij"), -1).reshape(-1, 3)
+    gpu = renderer.compile(g).probe(pts)
+    ref = oracle_mod.OracleGraph(g).de(pts, precision=32)
+    np.testing.assert_allclose(gpu["traps"][:, 0], ref["traps"][:, 0], rtol=0, atol=1e-6)
