@@ -1440,13 +1440,15 @@ extern "C" sf_status sf_graph_compile(sf_context* c, const sf_graph_desc* d, sf_
         g->d_inst = static_cast<float*>(p);
         g->prog.inst_data = reinterpret_cast<uint64_t>(g->d_inst);
     }
-    s = ctx_alloc(c, sizeof(DeProgram), &p);
+    g->prog_bytes = sizeof(DeProgram) * (interpreted(g->prog) ? 2 : 1);
+    s = ctx_alloc(c, g->prog_bytes, &p);
     if (s != SF_OK) {
         if (g->d_inst) ctx_free(c, g->d_inst, g->inst_bytes);
         delete g;
         return s;
     }
     g->d_prog = static_cast<DeProgram*>(p);
+    if (interpreted(g->prog)) g->d_next = g->d_prog + 1;
     cudaError_t e = cudaSuccess;
     if (g->d_inst) e = cudaMemcpyAsync(g->d_inst, inst.data(), g->inst_bytes, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
@@ -1454,7 +1456,7 @@ extern "C" sf_status sf_graph_compile(sf_context* c, const sf_graph_desc* d, sf_
     if (e == cudaSuccess && interpreted(g->prog)) e = sf_launch_prepare_program(g->d_prog, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
-        ctx_free(c, g->d_prog, sizeof(DeProgram));
+        ctx_free(c, g->d_prog, g->prog_bytes);
         if (g->d_inst) ctx_free(c, g->d_inst, g->inst_bytes);
         delete g;
         return cuda_fail(e, "graph upload");
@@ -1480,11 +1482,20 @@ extern "C" sf_status sf_graph_update(sf_graph* g, const sf_graph_desc* d) {
         return fail(SF_ERR_GRAPH, "topology changed: compile a new graph");
     P.inst_data = reinterpret_cast<uint64_t>(g->d_inst);
     cudaSetDevice(g->ctx->device);
+    // An interpreted program's ops are prepared apart: a launch that another thread makes
+    // meanwhile (a server's) finds the program of before or of after, never one whose ops
+    // still lack their constants, and an edit that fails here leaves the old one.
+    cudaStream_t st = g->ctx->stream;
+    if (g->d_next) {
+        CU(cudaMemcpyAsync(g->d_next, &P, sizeof P, cudaMemcpyHostToDevice, st));
+        CU(sf_launch_prepare_program(g->d_next, st));
+        CU(cudaStreamSynchronize(st));
+    }
     CU(cudaDeviceSynchronize());  // no launch on any stream (previews, server slots) may read what is replaced
-    if (g->d_inst) CU(cudaMemcpyAsync(g->d_inst, inst.data(), g->inst_bytes, cudaMemcpyHostToDevice, g->ctx->stream));
-    CU(cudaMemcpyAsync(g->d_prog, &P, sizeof P, cudaMemcpyHostToDevice, g->ctx->stream));
-    if (interpreted(P)) CU(sf_launch_prepare_program(g->d_prog, g->ctx->stream));
-    CU(cudaStreamSynchronize(g->ctx->stream));
+    if (g->d_inst) CU(cudaMemcpyAsync(g->d_inst, inst.data(), g->inst_bytes, cudaMemcpyHostToDevice, st));
+    if (g->d_next) CU(cudaMemcpyAsync(g->d_prog, g->d_next, sizeof P, cudaMemcpyDeviceToDevice, st));
+    else CU(cudaMemcpyAsync(g->d_prog, &P, sizeof P, cudaMemcpyHostToDevice, st));
+    CU(cudaStreamSynchronize(st));
     g->host = h;
     g->prog = P;
     g->info = info;
@@ -1505,7 +1516,7 @@ extern "C" sf_status sf_graph_destroy(sf_graph* g) {
     }
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
-    ctx_free(c, g->d_prog, sizeof(DeProgram));
+    ctx_free(c, g->d_prog, g->prog_bytes);
     if (g->d_inst) ctx_free(c, g->d_inst, g->inst_bytes);
     delete g;
     ctx_release(c);

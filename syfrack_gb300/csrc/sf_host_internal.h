@@ -94,6 +94,8 @@ struct sf_graph {
     sfh::HostGraph host;
     DeProgram prog;
     DeProgram* d_prog = nullptr;
+    DeProgram* d_next = nullptr;  // an edit's program until its ops are prepared (interpreted graphs)
+    size_t prog_bytes = 0;        // of d_prog and d_next, one block
     float* d_inst = nullptr;  // Instances blocks (DeProgram.inst_data)
     size_t inst_bytes = 0;
     sf_graph_info info;
