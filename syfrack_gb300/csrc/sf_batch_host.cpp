@@ -201,7 +201,11 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
     const size_t ex_bytes = rich ? size_t(paths) * 16 : 0;
     std::vector<const sf_graph*> graphs;
     for (uint32_t i = 0; i < n; ++i) graphs.push_back(jobs[i].graph);
-    const std::vector<uint32_t> keys = group_keys(graphs);
+    std::vector<uint32_t> keys;
+    {
+        const GraphLocks no_edit(graphs);
+        keys = group_keys(graphs);
+    }
     const uint32_t groups = uint32_t(std::set<uint32_t>(keys.begin(), keys.end()).size());
     sf_status st = arena_alloc(c, b->a, uint32_t(paths), n, rounds, K, groups,
                                scene_bytes + pv_bytes + ex_bytes + film_bytes, &extra);

@@ -1485,6 +1485,7 @@ extern "C" sf_status sf_graph_update(sf_graph* g, const sf_graph_desc* d) {
     // An interpreted program's ops are prepared apart: a launch that another thread makes
     // meanwhile (a server's) finds the program of before or of after, never one whose ops
     // still lack their constants, and an edit that fails here leaves the old one.
+    const std::lock_guard<std::mutex> edit(g->edit_mu);
     cudaStream_t st = g->ctx->stream;
     if (g->d_next) {
         CU(cudaMemcpyAsync(g->d_next, &P, sizeof P, cudaMemcpyHostToDevice, st));
@@ -1809,6 +1810,7 @@ extern "C" sf_status sf_session_dispatch(sf_session* s, sf_tile tile, uint32_t s
     cudaSetDevice(c->device);
     DispatchGeom g{tile.x, tile.y, tile.w, tile.h, tile.done, samples, uint32_t(paths), s->light_smem};
     cudaStream_t st = c->stream;
+    const std::lock_guard<std::mutex> no_edit(s->graph->edit_mu);
     if (s->cfg.integrator == SF_INTEGRATOR_MEGAKERNEL) {
         {
             // whole paths on persistent lanes (a composed world 290 -> 213 ms, a Mandelbox

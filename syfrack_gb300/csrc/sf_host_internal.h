@@ -5,8 +5,10 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -91,6 +93,10 @@ struct sf_context {
 struct sf_graph {
     sf_context* ctx = nullptr;
     int refs = 1;  // sessions hold a reference
+    // An edit replaces `prog` and the device program under it; a session's dispatch and a
+    // server's pass hold it while they read `prog` and launch, so that all the launches of a
+    // dispatch see one program and an edit's wait for the device covers them.
+    mutable std::mutex edit_mu;
     sfh::HostGraph host;
     DeProgram prog;
     DeProgram* d_prog = nullptr;
@@ -261,12 +267,25 @@ struct WaveArena {
     uint32_t min_blocks = 3, quantum = 128, regen = 4;
 };
 
+// Holds the edit_mu of several graphs, taken in one order by every caller.
+class GraphLocks {
+    std::vector<std::unique_lock<std::mutex>> held;
+
+public:
+    explicit GraphLocks(std::vector<const sf_graph*> graphs) {
+        std::sort(graphs.begin(), graphs.end(), std::less<const sf_graph*>());
+        graphs.erase(std::unique(graphs.begin(), graphs.end()), graphs.end());
+        for (const sf_graph* g : graphs) held.emplace_back(g->edit_mu);
+    }
+};
+
 // The trace groups of a batch's jobs by their graphs: one key per job (jobs of one key
 // share a group; sort the table by it). A key is a form and the variant of its iteration
 // that the form's routine chooses (the trap, the fold's clamp), so that the lanes of a
 // warp choose alike; with more than SF_MAX_GROUPS of those, the form alone. Every group
 // costs its warps a wait for their longest segments, so what a batch can run in one
 // routine stays in one group: a Mandelbox pair of scales 2 and -2 took 7.1 ms as two.
+// The caller holds the graphs' edit_mu (GraphLocks).
 std::vector<uint32_t> group_keys(const std::vector<const sf_graph*>& graphs);
 // Adds a job to the table being built, in key order: returns its group, which starts at
 // path_begin if the job opens it.

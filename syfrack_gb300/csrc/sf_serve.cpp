@@ -327,6 +327,7 @@ sf_status launch_wave(sf_server* s, ServeSlot& sl) {
     // the job table sorted by group (the requests keep their order: a film's passes)
     std::vector<const sf_graph*> graphs;
     for (const ServeReq* r : sl.reqs) graphs.push_back(r->film->graph);
+    const GraphLocks no_edit(graphs);
     const std::vector<uint32_t> keys = group_keys(graphs);
     std::vector<uint32_t> order(sl.reqs.size());
     for (uint32_t i = 0; i < order.size(); ++i) order[i] = i;

@@ -73,3 +73,55 @@ def test_served_frames_during_edits_to_the_same_values(renderer):
         for _ in range(150):
             np.testing.assert_array_equal(frame(), want)
     srv.close()
+
+
+@pytest.mark.parametrize("integrator", ["wavefront", "megakernel"])
+def test_dispatches_during_value_edits(renderer, integrator):
+    """A session's frames while another thread switches its Mandelbox between two sets of
+    values (fold limit, scale and trap scale): each is one set's frame, bit for bit."""
+    scene = workloads.mandelbox_scene()
+    scene.graph = workloads.mandelbox_graph(scale=-1.6)  # a handle of its own
+    other = workloads.mandelbox_graph(scale=-2.0)
+    for n in other.nodes:
+        if n.kind.name == "BoxFold":
+            n.kind.fields["limit"] = 0.8
+        elif n.kind.name == "Trap":
+            n.kind.fields["scale"] = 0.5
+    cg = renderer.compile(scene.graph)
+    cfg = RenderConfig(width=64, height=48, samples_per_pixel=1, max_bounces=3, max_steps=128, tile_size=64,
+                       samples_per_dispatch=1, integrator=integrator)
+    s = RenderSession(renderer, scene, cfg)
+    kept = {}
+
+    def frame():
+        s.dispatch((0, 0, 64, 48, 0), 1)
+        assert s.sync() == 0
+        return s.readback().accum
+
+    # one sample more is added to the film by every dispatch of sample 0: differences are frames
+    def edit(g):
+        desc, kept[0] = g.to_desc()
+        assert cg.ctx.lib.sf_graph_update(cg.h, C.byref(desc)) == 0
+
+    last = np.zeros((48, 64, 4), np.float32)
+    want = []
+    for g in (scene.graph, other):
+        edit(scene.graph)  # every session takes the march's constants from the first set
+        fresh = RenderSession(renderer, scene, cfg)
+        edit(g)
+        fresh.dispatch((0, 0, 64, 48, 0), 1)
+        assert fresh.sync() == 0
+        want.append(fresh.readback().accum)
+        fresh.close()
+    assert not np.array_equal(want[0], want[1])
+    seen = set()
+    with edited(cg, [scene.graph, other]):
+        for _ in range(200):
+            now = frame()
+            match = [k for k in (0, 1) if np.array_equal(now, last + want[k])]
+            assert match
+            seen.add(match[0])
+            last = now
+    edit(scene.graph)
+    s.close()
+    assert seen == {0, 1}
