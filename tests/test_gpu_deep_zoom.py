@@ -121,3 +121,22 @@ def test_budgets_around_the_chunk(gpu_ctx, max_iter):
     assert (a["iterations"] == a["iterations_f64"]).mean() >= 0.99
     for k in ("iterations", "smooth", "rebases"):
         np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+@pytest.mark.parametrize("max_iter", [59, 60, 61, 700])
+@pytest.mark.parametrize("centre,width", [((0.5, 0.6), 3.0), ((-0.75, 0.1), 0.3), ((-0.75, 0.1), 0.01),
+                                          ((0.27868532354762443, 0.5820921261345181), 0.01)])
+def test_dense_rebases(gpu_ctx, centre, width, max_iter):
+    """Views whose pixels rebase every few iterations (a reference that escapes after 5 or
+    33 iterations, offsets of the orbit's own size), where warps leave the chunks for runs
+    of 60 checked iterations and come back. Counts differ from FP64 direct iteration only
+    where binary32's rounding, grown by the orbit, decides the last step."""
+    args = dict(center_hi=centre, center_lo=(0.0, 0.0), width_units=width, width=131, height=93, max_iter=max_iter)
+    a = deep_zoom(gpu_ctx, **args, reference_f64=True)
+    b = deep_zoom(gpu_ctx, **args, orbit="host")
+    inside = a["iterations_f64"] < max_iter
+    # an offset grows by 2 |z| an iteration, so long orbits lose more of the 24 bits
+    assert (a["iterations"] == a["iterations_f64"]).mean() >= (0.99 if max_iter <= 61 else 0.95)
+    assert inside.any() and a["rebases"] >= 131 * 93 * (1 if width >= 0.3 else 0)
+    for k in ("iterations", "smooth", "rebases"):
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
