@@ -121,6 +121,21 @@ static __device__ __forceinline__ float sin_multiple(float c, float s, int k) {
     return sign * b;
 }
 
+// The same at 12 stripes, unrolled (bit for bit): power 2 off the z^2 loop, which twisted
+// tiles at the default stripes take. A Mandelbrot tile of 1024x1024, 4,000 iterations,
+// twist 10: 2.03 ms with the loop, 1.16 so.
+static __device__ __forceinline__ float sin_multiple_12(float c, float s) {
+    const float c2 = 2.0f * c;
+    float a = 0.0f, b = s;
+#pragma unroll
+    for (int j = 1; j < 12; ++j) {
+        const float t = fmaf(c2, b, -a);
+        a = b;
+        b = t;
+    }
+    return b;
+}
+
 // sin(12 theta) / 4, the default stripe count of PlanarFractal, from the double angle:
 // with C = cos 2 theta and h = sin(2 theta) / 2, sin 3u = sin u (3 - 4 sin^2 u) and
 // cos 3u = cos u (1 - 4 sin^2 u) at u = 2 theta give
@@ -133,9 +148,9 @@ static __device__ __forceinline__ float quarter_sin_12(float C, float h, float s
 }
 
 // One iteration; true once the orbit has escaped or spent its iteration budget.
-// POW2: the power is 2 (z^2 as one complex square).
+// POW2: the power is 2 (z^2 as one complex square). SK12: the stripe count is 12.
 // o.stripe accumulates sin(k theta); the bands use 0.5 n + 0.5 * that sum.
-template <bool TRAPS, bool POW2>
+template <bool TRAPS, bool POW2, bool SK12 = false>
 static __device__ __forceinline__ bool esc_step(const EscParams& p, EscOrbit& o) {
     if (o.count >= p.iterations) return true;
     float r2 = FA(FM(o.zx, o.zx), FM(o.zy, o.zy));
@@ -149,7 +164,8 @@ static __device__ __forceinline__ bool esc_step(const EscParams& p, EscOrbit& o)
         o.ring = fminf(o.ring, fabsf(radius - p.trap_radius));
         float s = 0.0f;
         if (r2 > 0.0f) {
-            if (p.stripe_k != SF_STRIPES_GENERAL) s = sin_multiple(o.zx * rinv, o.zy * rinv, p.stripe_k);
+            if (SK12) s = sin_multiple_12(o.zx * rinv, o.zy * rinv);
+            else if (p.stripe_k != SF_STRIPES_GENERAL) s = sin_multiple(o.zx * rinv, o.zy * rinv, p.stripe_k);
             else s = sinf(p.stripes * atan2f(o.zy, o.zx));
         }
         o.stripe += s;
@@ -374,7 +390,7 @@ __global__ void __launch_bounds__(256) k_escape2d_root(const PlanarDev* __restri
 // lanes at once.
 // Without TRAPS only dist, traps[0 .. n) (smooth time) and iters are written.
 constexpr int ESC_CHUNK = 16, ESC_REGEN = 8, ESC_WAIT = 4;
-enum { ESC_GENERAL = 0, ESC_POW2 = 1, ESC_Z2 = 2, ESC_SHIP = 3, ESC_PHOENIX = 4 };
+enum { ESC_GENERAL = 0, ESC_POW2 = 1, ESC_POW2_12 = 2, ESC_Z2 = 3, ESC_SHIP = 4, ESC_PHOENIX = 5 };
 
 // One iteration of z^2 without twist at the default 12 stripes: Julia and Mandelbrot
 // (ESC_Z2), Burning Ship, Phoenix. r2 = |z|^2 of the point it leaves; the caller has
@@ -476,7 +492,7 @@ template <bool TRAPS, int MODE>
 static __device__ __forceinline__ bool esc_advance(const EscParams& p, EscOrbit& o) {
     if (MODE >= ESC_Z2) return esc_chunk_z2<TRAPS, MODE>(p, o);
     for (int j = 0; j < ESC_CHUNK; ++j)
-        if (esc_step<TRAPS, MODE == ESC_POW2>(p, o)) return true;
+        if (esc_step<TRAPS, MODE != ESC_GENERAL, MODE == ESC_POW2_12>(p, o)) return true;
     return false;
 }
 
@@ -542,14 +558,15 @@ __global__ void __launch_bounds__(256, 4) k_escape2d(const PlanarDev* __restrict
     __syncthreads();
     const uint32_t n = tile_w * tile_h;
     const EscParams p = esc_params(F);
-    // the z^2 loop: 12 stripes, no twist, and a bailout whose |z|^2 stays finite, so that
-    // an orbit has passed it before any product overflows
-    const bool z2 = p.power == 2 && p.stripe_k == 12 && !p.rotate && p.bail_t <= 1e37f;
+    // the z^2 loop: 12 stripes, no twist, and a bailout below which 2 |x y| <= |z|^2 is
+    // finite, so that an orbit has passed it before any product overflows
+    const bool z2 = p.power == 2 && p.stripe_k == 12 && !p.rotate && p.bail_t <= 1.6e38f;
     unsigned long long total;
 #define ESC_RUN(MODE) esc_pixels<TRAPS, MODE>(F, K, p, tile_x, tile_y, tile_w, n, sample, dist, traps, iters, work)
     if (z2 && p.ship) total = ESC_RUN(ESC_SHIP);
     else if (z2 && p.phoenix) total = ESC_RUN(ESC_PHOENIX);
     else if (z2) total = ESC_RUN(ESC_Z2);
+    else if (p.power == 2 && p.stripe_k == 12) total = ESC_RUN(ESC_POW2_12);
     else if (p.power == 2) total = ESC_RUN(ESC_POW2);
     else total = ESC_RUN(ESC_GENERAL);
 #undef ESC_RUN
