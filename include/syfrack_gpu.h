@@ -655,8 +655,8 @@ typedef struct sf_server_config {
     uint32_t max_jobs;          /* requests per batch, 1..1024                        */
     uint32_t max_tile_pixels;   /* 2D pixels per batch                                */
     uint32_t min_blocks, quantum, regen; /* trace launch shape (sf_batch_set_launch);
-                                          * a batch of 2M paths or fewer is not split by
-                                          * the quantum                               */
+                                          * quantum 0: 128, and none for a batch of
+                                          * 2M paths or fewer                         */
     uint32_t pad;
 } sf_server_config;
 typedef struct sf_request {
@@ -695,8 +695,8 @@ typedef struct sf_server_stats {
     double now_ms;
 } sf_server_stats;
 /* Starts the scheduler thread. Defaults for zero fields: 4 slots, 4M paths, 256 jobs,
- * 32M tile pixels, 1 GiB of host results, launch shape 3 blocks/SM, quantum 128 and
- * regeneration threshold 4. */
+ * 32M tile pixels, 1 GiB of host results, launch shape 3 blocks/SM, quantum 128
+ * (none for a batch of 2M paths or fewer) and regeneration threshold 4. */
 sf_status sf_server_create(sf_context* ctx, const sf_server_config* cfg, sf_server** out);
 /* Queues a request; returns at once with its ticket (tickets start at 1). */
 sf_status sf_serve_submit(sf_server* s, const sf_request* req, uint64_t* ticket);

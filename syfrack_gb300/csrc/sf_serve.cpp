@@ -166,11 +166,13 @@ struct ServeReq {
 };
 
 constexpr uint32_t kServeMaxSlots = 8;
-// A batch of up to this many paths (about 18 for each lane of 3 blocks an SM) marches its
-// segments in one launch a round whatever the step quantum: the launches that only carry
-// on at a quantum cost it more than the shorter tails give. One 480x270 preview 2.25 ms
+// A server without a step quantum of its own splits at kServeQuantum, but a batch of up to
+// kServeUnsplitPaths paths (about 18 for each lane of 3 blocks an SM) marches its segments in
+// one launch a round: the launches that only carry on at a quantum cost it more than the
+// shorter tails give. A caller's quantum bounds the launches of every batch, whatever its
+// size. One 480x270 preview 2.25 ms
 // with quanta of 128 steps and 1.91 without, 8 previews and 4 refinements 16.7 and 15.3.
-constexpr uint32_t kServeUnsplitPaths = 1u << 21;
+constexpr uint32_t kServeQuantum = 128, kServeUnsplitPaths = 1u << 21;
 constexpr uint32_t kServeShadowSlots = 3;  // shadow segments per bounce the slot arenas hold
 constexpr uint32_t kServeMaxTiles = 64;  // 2D tiles per batch
 // A tile's device block starts with PlanarDev (0), CanvasDev (256) and its pixel
@@ -194,6 +196,7 @@ struct ServeSlot {
 struct sf_server {
     sf_context* ctx = nullptr;
     sf_server_config cfg{};
+    bool own_quantum = false;  // the caller set no step quantum
     ServeClock::time_point t0;
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
@@ -373,7 +376,7 @@ sf_status launch_wave(sf_server* s, ServeSlot& sl) {
     WaveArena pass = a;
     pass.rounds = rounds;
     pass.groups = a.bt.groups;  // and its groups
-    if (paths <= kServeUnsplitPaths) pass.quantum = 0;
+    if (s->own_quantum && paths <= kServeUnsplitPaths) pass.quantum = 0;
     // scenes with finish details, a texture or optics: the feature-built kernels and the
     // footprint and medium rows (kept by the slot, unused by plain batches)
     pass.rich = rich;
@@ -569,7 +572,8 @@ extern "C" sf_status sf_server_create(sf_context* c, const sf_server_config* cfg
     if (!k.max_tile_pixels) k.max_tile_pixels = 1u << 25;
     if (!k.host_result_bytes) k.host_result_bytes = uint64_t(1) << 30;
     if (!k.min_blocks) k.min_blocks = 3;
-    if (!k.quantum) k.quantum = 128;
+    const bool own_quantum = k.quantum == 0;
+    if (own_quantum) k.quantum = kServeQuantum;
     if (!k.regen) k.regen = 4;
     if (!k.hbm_budget) return fail(SF_ERR_INVALID, "hbm_budget must be set");
     if (k.slots > kServeMaxSlots) return fail(SF_ERR_INVALID, "1..8 slots");
@@ -581,6 +585,7 @@ extern "C" sf_status sf_server_create(sf_context* c, const sf_server_config* cfg
     auto* s = new sf_server();
     s->ctx = c;
     s->cfg = k;
+    s->own_quantum = own_quantum;
     s->pool.budget = k.hbm_budget;
     ctx_retain(c);
     auto bail = [&](sf_status st) {

@@ -53,11 +53,12 @@ class ServeResult:
 class Server:
     """A serving loop on one device (sf_server_create). hbm_budget bounds the
     device bytes of films and tile outputs held at once; requests wait in the queue
-    until they fit."""
+    until they fit. quantum: the march steps a segment takes in one trace launch, for
+    every batch; 0 = 128, and no bound for batches of 2M paths or fewer."""
 
     def __init__(self, renderer: Renderer, hbm_budget: int, slots: int = 4, path_capacity: int = 1 << 22,
                  max_jobs: int = 256, max_tile_pixels: int = 1 << 25, host_result_bytes: int = 1 << 30,
-                 min_blocks: int = 3, quantum: int = 128, regen: int = 4):
+                 min_blocks: int = 3, quantum: int = 0, regen: int = 4):
         self.renderer = renderer
         self.ctx = renderer.ctx
         k = sf_server_config(hbm_budget=hbm_budget, host_result_bytes=host_result_bytes, slots=slots,

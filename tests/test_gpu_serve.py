@@ -217,3 +217,23 @@ def test_sky_lit_preview_served(renderer):
     with pytest.raises(SyfrackError, match="SF_ERR_UNSUPPORTED"):
         srv.preview(sc, cfg)
     srv.close()
+
+
+@pytest.mark.parametrize("quantum", [8, 64])
+def test_callers_quantum_bounds_small_batches(renderer, quantum):
+    """A step quantum that the caller sets splits every batch's rounds, small ones too
+    (more launches than without one), and the films stay the same bit for bit: one preview
+    with its refinement, then a batch of several forms."""
+    films, launches = [], []
+    for q in (0, quantum):
+        srv = Server(renderer, hbm_budget=2 * GB, slots=1, quantum=q)
+        first = srv.preview(*small_preview(0))
+        out = [srv.wait(first).accum, srv.wait(srv.refine(first, 3)).accum]
+        launches.append(srv.stats()["launches"])
+        mix = [srv.preview(*small_preview(i)) for i in range(1, 9)]
+        out += [srv.wait(t).accum for t in mix]
+        films.append(out)
+        srv.close()
+    assert launches[1] > launches[0]
+    for a, b in zip(*films):
+        np.testing.assert_array_equal(a, b)
