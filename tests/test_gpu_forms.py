@@ -6,7 +6,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from helpers import bounded_bulb
+from helpers import bounded_bulb, golden_scene
 from syfrack_gb300 import Batch, RenderSession
 from syfrack_gb300.graph import Graph
 from syfrack_gb300.scene import AreaLight, Camera, Material, RenderConfig, Scene
@@ -101,4 +101,49 @@ def test_batch_groups(renderer, picks):
         s.close()
         np.testing.assert_array_equal(got.depth, ref.depth, err_msg=str(VARIANTS[picks[i]]))
         np.testing.assert_array_equal(got.accum, ref.accum, err_msg=str(VARIANTS[picks[i]]))
+    b.close()
+
+
+# Batches of several groups: more variants than groups; scenes with one and with three
+# shadow slots (area lights, then a sun and a sky) over four forms.
+def launch_shape_jobs(kind):
+    light = AreaLight(position=(1.0, 3.5, -3.5), normal=(-1.0, -3.5, 3.5), size=(1.0, 1.0), intensity=10.0)
+    scenes = []
+    for i, k in enumerate(range(10) if kind == "variants" else (1, 2, 7)):
+        form, trap, params = VARIANTS[k]
+        scenes.append(Scene(graph=graph_of(form, trap, **params), camera=camera_of(form),
+                            material=Material(albedo=(0.7, 0.7, 0.7), roughness=0.2, metallic=0.0, specular=0.04),
+                            lights=[light], seed=5 + i))
+    if kind == "slots":
+        scenes += [golden_scene("menger"), golden_scene("mandelbulb")]
+    return [(sc, RenderConfig(21 + 7 * i, 17 + i, 2, max_bounces=3, max_steps=256, pixel_tolerance=1.0, tile_size=128,
+                              samples_per_dispatch=2, integrator="wavefront")) for i, sc in enumerate(scenes)]
+
+
+@pytest.fixture(scope="module", params=["variants", "slots"])
+def jobs_alone(renderer, request):
+    jobs, films = launch_shape_jobs(request.param), []
+    for sc, cfg in jobs:
+        s = RenderSession(renderer, sc, cfg)
+        while not s.step(0):
+            pass
+        films.append(s.readback())
+        s.close()
+    return jobs, films
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+@pytest.mark.parametrize("shape", [(3, 16, 4), (2, 8, 1), (4, 128, 32), (4, 0, 8)])
+def test_batch_launch_shapes(renderer, jobs_alone, shape, use_graph):
+    """Segments cut at a step quantum and resumed, group by group, launched one by one and
+    replayed as a graph: every film is the job's alone, bit for bit."""
+    jobs, films = jobs_alone
+    b = Batch(renderer, jobs)
+    b.set_launch(*shape)
+    b.run(1, use_graph=use_graph)
+    assert b.sync() == 0
+    for i, ref in enumerate(films):
+        got = b.readback(i)
+        np.testing.assert_array_equal(got.depth, ref.depth, err_msg=str(i))
+        np.testing.assert_array_equal(got.accum, ref.accum, err_msg=str(i))
     b.close()
