@@ -701,7 +701,8 @@ sf_status ctx_alloc(sf_context* c, size_t bytes, void** p, bool trim) {
         c->cached.erase(c->cached.begin());
     }
     if (trim && c->used + bytes > c->budget) {
-        // The cached scratch of primary and escape-time calls gives way to an admission.
+        // The cached scratch (of probes, primary rays, escape time and deep zoom) gives way to
+        // an admission.
         // Its owner (stage_mu) may be in a readback: then wait for it, taking the locks in
         // the order the scratch's users take them (stage_mu, then alloc_mu), so that the
         // admission's outcome does not depend on timing. No caller that trims holds stage_mu.
@@ -871,6 +872,37 @@ sf_status ensure_scratch(sf_context* c, size_t bytes) {
     if (s == SF_OK) c->scratch_bytes = bytes;
     return s;
 }
+
+// Device memory of one call: up to kScratchKept bytes the context's scratch, kept for the
+// next call, above that an allocation of the call's own, so that no call leaves more than
+// that behind. Holds stage_mu from take() on.
+constexpr size_t kScratchKept = size_t(512) << 20;
+class CallMemory {
+    sf_context* c;
+    std::unique_lock<std::mutex> lk;
+    void* own = nullptr;
+    size_t own_bytes = 0;
+
+public:
+    char* p = nullptr;
+    explicit CallMemory(sf_context* ctx) : c(ctx), lk(ctx->stage_mu, std::defer_lock) {}
+    ~CallMemory() { ctx_free(c, own, own_bytes); }
+    CallMemory(const CallMemory&) = delete;
+    CallMemory& operator=(const CallMemory&) = delete;
+    sf_status take(size_t bytes) {
+        if (bytes > kScratchKept) {
+            if (const sf_status s = ctx_alloc(c, bytes, &own); s != SF_OK) return s;
+            own_bytes = bytes;
+            lk.lock();
+            p = static_cast<char*>(own);
+            return SF_OK;
+        }
+        lk.lock();
+        if (const sf_status s = ensure_scratch(c, bytes); s != SF_OK) return s;
+        p = static_cast<char*>(c->scratch);
+        return SF_OK;
+    }
+};
 
 std::string topology_of(const HostGraph& g) {
     // Everything but the float parameters (topology_key, graph/mod.rs:397-425).
@@ -1543,12 +1575,12 @@ extern "C" sf_status sf_de_probe(sf_graph* g, const float* xyz, size_t n, sf_de_
     sf_context* c = g->ctx;
     cudaSetDevice(c->device);
     static_assert(sizeof(sf_de_sample) == 28, "distance, traps, iterations and material, packed");
-    // points and samples as the caller holds them, in the context's scratch
-    std::lock_guard<std::mutex> lk(c->stage_mu);
+    // points and samples as the caller holds them
     const size_t in_bytes = (n * 12 + 255) & ~size_t(255);
-    if (const sf_status s = ensure_scratch(c, in_bytes + n * sizeof(sf_de_sample)); s != SF_OK) return s;
-    float* d_in = static_cast<float*>(c->scratch);
-    float* d_out = reinterpret_cast<float*>(static_cast<char*>(c->scratch) + in_bytes);
+    CallMemory mem(c);
+    if (const sf_status s = mem.take(in_bytes + n * sizeof(sf_de_sample)); s != SF_OK) return s;
+    float* d_in = reinterpret_cast<float*>(mem.p);
+    float* d_out = reinterpret_cast<float*>(mem.p + in_bytes);
     cudaError_t e = cudaMemcpyAsync(d_in, xyz, n * 12, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
         LaunchTimer t(c, true);
@@ -2390,16 +2422,9 @@ extern "C" sf_status sf_deep_zoom(sf_context* c, const sf_deep_zoom_desc* d, uin
     const size_t Zb = d->orbit_mode == SF_ORBIT_DEVICE ? ((M * 16 + 255) & ~size_t(255)) : 0;
     const size_t z_off = (2 * Mb + 256 + n * 8 * (reference_f64 ? 2 : 1) + 255) & ~size_t(255);
     size_t bytes = z_off + Zb;
-    // the context's scratch, kept between calls, for frames up to 8K; larger ones allocate
-    const bool kept = bytes <= (size_t(512) << 20);
-    std::unique_lock<std::mutex> lk(c->stage_mu, std::defer_lock);
-    if (kept) lk.lock();
-    void* buf = nullptr;
-    sf_status st = kept ? ensure_scratch(c, bytes) : ctx_alloc(c, bytes, &buf);
-    if (st != SF_OK) return st;
-    if (kept) buf = c->scratch;
-    else lk.lock();
-    char* b = static_cast<char*>(buf);
+    CallMemory mem(c);  // kept for frames up to 8K
+    if (const sf_status s = mem.take(bytes); s != SF_OK) return s;
+    char* const b = mem.p;
     float2* olo = reinterpret_cast<float2*>(b);
     float2* of = reinterpret_cast<float2*>(b + Mb);
     uint32_t* olen = reinterpret_cast<uint32_t*>(b + 2 * Mb);  // orbit length | pixel counter
@@ -2461,9 +2486,7 @@ extern "C" sf_status sf_deep_zoom(sf_context* c, const sf_deep_zoom_desc* d, uin
     unsigned long long after[SF_STAT_COUNT];
     if (e == cudaSuccess) e = cudaMemcpyAsync(after, c->d_stats, sizeof after, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (!kept) ctx_free(c, buf, bytes);
     if (e != cudaSuccess) return cuda_fail(e, "sf_deep_zoom");
-    lk.unlock();
     if (rebases) *rebases = after[SF_STAT_STEPS] - before[SF_STAT_STEPS];
     return SF_OK;
 }

@@ -77,8 +77,9 @@ struct sf_context {
     int refs = 1;
     std::mutex mu;
     std::mutex alloc_mu;  // budget accounting (a server thread allocates too)
-    // pinned staging of readbacks and the primary-ray scratch, grown on demand and
-    // reused by every call (stage_mu guards both)
+    // pinned staging of a host orbit's upload, and the device scratch of probes, primary
+    // rays, escape time and deep zoom: grown on demand and reused by every call (stage_mu
+    // guards both)
     void* stage = nullptr;
     size_t stage_bytes = 0;
     void* scratch = nullptr;
@@ -110,9 +111,8 @@ struct sf_graph {
 
 namespace sfh {
 
-// Device memory under the context's HBM admission budget.
-// Device memory within the context's budget; `trim` lets the cached scratch of
-// primary and escape-time calls be released first (callers holding stage_mu pass false).
+// Device memory within the context's HBM admission budget; `trim` lets the cached scratch
+// be released first (callers holding stage_mu pass false).
 sf_status ctx_alloc(sf_context* c, size_t bytes, void** p, bool trim = true);
 void ctx_free(sf_context* c, void* p, size_t bytes);
 // Frees an idle block into the context's cache of session arenas (at most four).

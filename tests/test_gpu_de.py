@@ -222,3 +222,24 @@ def test_mixed_batch_scale_band_the_reference_rejects(renderer):
     scales = [n.kind.fields["factor"] for sc, _ in jobs for n in sc.graph.nodes if n.kind.name == "Scale"]
     assert len(scales) >= 20 and min(abs(x) for x in scales) >= 1e-3
     assert min(scales) < -1.0 and max(scales) > 1.0 and any(abs(x) < 1.05 for x in scales)
+
+
+@pytest.mark.parametrize("n", [1, 4097, 13_500_000])  # 40 bytes a point: the last is past 512 MB
+def test_probe_memory_kept(n):
+    """A probe leaves at most 512 MB behind, nothing of a larger one, and samples do not
+    depend on whose memory they were computed in."""
+    from syfrack_gb300 import GpuContext, Renderer
+
+    ctx = GpuContext()
+    g = Renderer(ctx).compile(Graph.bundled("sphere"))
+    few = np.random.default_rng(3).uniform(-2, 2, (1000, 3)).astype(np.float32)
+    used = ctx.memory()[0]
+    r = g.probe(np.resize(few, (n, 3)))
+    kept = ctx.memory()[0] - used
+    assert kept == 0 if 40 * n > 512 << 20 else 40 * n <= kept <= 40 * n + 256
+    ref = g.probe(few)
+    for k in ref:
+        m = min(n, 1000)
+        np.testing.assert_array_equal(r[k][:m], ref[k][:m])
+        np.testing.assert_array_equal(r[k][-1], ref[k][(n - 1) % 1000])
+    ctx.close()
