@@ -382,7 +382,8 @@ typedef struct sf_primary_desc {
 } sf_primary_desc;
 sf_status sf_primary_trace(sf_graph* graph, const sf_primary_desc* desc, float* t_out, uint32_t* steps_out,
                            float* normal_out);
-/* Same, with the normals as (pixel, 3) rows in normal_out. */
+/* Same, with the normals as (pixel, 3) rows in normal_out. Added within ABI 1.6, which it
+ * leaves as it is: a caller that may meet an older library looks the symbol up. */
 sf_status sf_primary_trace_rows(sf_graph* graph, const sf_primary_desc* desc, float* t_out, uint32_t* steps_out,
                                 float* normal_out);
 
