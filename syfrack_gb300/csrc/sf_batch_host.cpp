@@ -258,8 +258,7 @@ extern "C" sf_status sf_batch_create(sf_context* c, const sf_batch_job* jobs, ui
         j.geom = DispatchGeom{0, 0, cf.width, cf.height, 0, spd, uint32_t(px * spd)};
         j.path_begin = pbeg;
         j.pixel_begin = xbeg;
-        j.form = jobs[i].graph->prog.form;
-        j.group = group_of(b->a.bt, last_key, keys[i], j.form, pbeg);
+        j.group = group_of(b->a.bt, last_key, keys[i], jobs[i].graph->prog.form, pbeg);
         pbeg += uint32_t(px * spd);
         xbeg += uint32_t(px);
         b->slot[i] = uint32_t(b->jobs.size());
@@ -391,7 +390,7 @@ extern "C" sf_status sf_batch_readback(sf_batch* b, uint32_t job, sf_film_planes
     if (job >= b->jobs.size()) return fail(SF_ERR_INVALID, "job index out of range");
     sf_context* c = b->ctx;
     cudaSetDevice(c->device);
-    CU(film_readback(c, b->jobs[b->slot[job]].film, *out, c->stream));
+    CU(film_readback(b->jobs[b->slot[job]].film, *out, c->stream));
     return SF_OK;
 }
 

@@ -202,27 +202,8 @@ __device__ __forceinline__ void spherical_power(float3 p, float r, uint32_t n, f
     deriv = float(n) * prev;
 }
 
-// The Power node's trigonometric path (non-integer exponents, radii below 1e-12): the
-// unit direction, its radius and the factor of dr.
-struct PowerTrig {
-    float3 dir;
-    float zr, factor;
-};
-__device__ __forceinline__ PowerTrig power_trig(float3 p, float radius, float power) {
-    PowerTrig o;
-    float r = fmaxf(radius, 1e-12f);
-    float theta = radius >= 1e-12f ? atan2f(sqrtf(fmaf(p.x, p.x, p.y * p.y)), p.z)
-                                   : acosf(fminf(fmaxf(p.z / r, -1.0f), 1.0f));
-    float phi = atan2f(p.y, p.x);
-    o.factor = powf(r, power - 1.0f) * power;
-    o.zr = powf(r, power);
-    float st, ct, sp, cp;
-    sincosf(theta * power, &st, &ct);
-    sincosf(phi * power, &sp, &cp);
-    o.dir = mk3(st * cp, st * sp, ct);
-    return o;
-}
-// Power node (eval.rs:456-476).
+// Power node (eval.rs:456-476), including the trigonometric path for
+// non-integer exponents and radii below 1e-12.
 __device__ __forceinline__ void power_op(float3& p, float& dr, float radius, float power, uint32_t power_int) {
     if (radius >= 1e-12f && power_int != 0) {
         float3 q;
@@ -232,9 +213,16 @@ __device__ __forceinline__ void power_op(float3& p, float& dr, float radius, flo
         dr *= dv;
         return;
     }
-    const PowerTrig q = power_trig(p, radius, power);
-    dr *= q.factor;
-    p = q.dir * q.zr;
+    float r = fmaxf(radius, 1e-12f);
+    float theta = radius >= 1e-12f ? atan2f(sqrtf(fmaf(p.x, p.x, p.y * p.y)), p.z)
+                                   : acosf(fminf(fmaxf(p.z / r, -1.0f), 1.0f));
+    float phi = atan2f(p.y, p.x);
+    dr *= powf(r, power - 1.0f) * power;
+    float zr = powf(r, power);
+    float st, ct, sp, cp;
+    sincosf(theta * power, &st, &ct);
+    sincosf(phi * power, &sp, &cp);
+    p = mk3(st * cp, st * sp, ct) * zr;
 }
 
 __device__ __forceinline__ float bulb_fence(float3 p, float dr) {
@@ -299,18 +287,6 @@ __device__ __forceinline__ float2 mul2(float ax, float ay, float bx, float by) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(ax), "f"(ay));
     asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(bx), "f"(by));
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(rd));
-    return r;
-}
-
-// (a.x + b.x, a.y + b.y) as one packed add (add.rn.f32x2): each lane rounds as a
-// binary32 add.
-__device__ __forceinline__ float2 add2(float ax, float ay, float bx, float by) {
-    unsigned long long ra, rb, rd;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(ax), "f"(ay));
-    asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(bx), "f"(by));
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
     float2 r;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(rd));
     return r;

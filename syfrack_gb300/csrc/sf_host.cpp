@@ -1993,8 +1993,7 @@ namespace sfh {
 // (RenderOutput.color); a film without the volume layer split (no fog) has a zero volume
 // contribution: volume and moments are (0, 0, 0, samples) and surface = accum. These
 // planes receive accum and are derived in place by the host threads.
-cudaError_t film_readback(sf_context* c, const FilmPlanes& f, const sf_film_planes& out, cudaStream_t st) {
-    (void)c;
+cudaError_t film_readback(const FilmPlanes& f, const sf_film_planes& out, cudaStream_t st) {
     const size_t px = size_t(f.width) * f.height;
     const bool split = f.vol != nullptr;
     populate_pages({{out.accum, px * 16}, {out.depth, px * 4}, {out.aux, px * 16}, {out.volume, px * 16},
@@ -2036,7 +2035,7 @@ extern "C" sf_status sf_session_readback(sf_session* s, sf_film_planes* out) {
     if (!s || !out) return fail(SF_ERR_INVALID, "null argument");
     sf_context* c = s->ctx;
     cudaSetDevice(c->device);
-    CU(film_readback(c, s->film, *out, c->stream));
+    CU(film_readback(s->film, *out, c->stream));
     return SF_OK;
 }
 

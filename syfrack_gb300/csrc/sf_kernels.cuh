@@ -161,7 +161,6 @@ struct BatchJob {
     DispatchGeom geom;
     uint32_t path_begin;
     uint32_t pixel_begin;
-    uint32_t form;
     uint32_t group;  // of BatchTable
 };
 #define SF_BATCH_MAX_JOBS 1024

@@ -348,8 +348,7 @@ sf_status launch_wave(sf_server* s, ServeSlot& sl) {
         j.geom = DispatchGeom{0, 0, r->width, r->height, r->sample_start, r->samples, px * r->samples};
         j.path_begin = paths;
         j.pixel_begin = pixels;
-        j.form = f->graph->prog.form;
-        j.group = group_of(a.bt, last_key, keys[order[i]], j.form, paths);
+        j.group = group_of(a.bt, last_key, keys[order[i]], f->graph->prog.form, paths);
         hj[i] = j;
         paths += px * r->samples;
         pixels += px;
