@@ -2,7 +2,7 @@
 // variant), so a warp's lanes run one form's code. A warp that finds a group's items
 // taken goes on to the next group's while others finish theirs, so the groups share one
 // launch and one tail. With the form chosen per lane in one loop, 64 mixed jobs took
-// 105 ms a pass (4 blocks per SM, no quantum, regeneration 8) and 67 this way.
+// 105 ms a pass (4 blocks per SM, no quantum, regeneration 8) and 60 this way.
 // GENERIC: the batch has a group of generic graphs (the interpreter's stack and calls).
 #pragma once
 #include "sf_trace_kernel.cuh"

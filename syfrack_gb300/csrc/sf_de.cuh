@@ -844,7 +844,9 @@ __device__ __forceinline__ bool inst_next(InstFrame& F) {
 // Evaluation modes of the generic interpreter.
 enum : uint32_t {
     SF_EVAL_FAST = 0,   // de_sample: skippable branches skipped outside their margin, the sample flagged
-    SF_EVAL_EXACT = 1,  // de_sample_exact: every branch evaluated
+    // de_sample_exact: every branch that can be the sample evaluated (a Union's second operand
+    // whose lower bound reaches a first operand that waits for it cannot: out_of_reach)
+    SF_EVAL_EXACT = 1,
     // the union probe (graph_wgsl.rs:1124-1136, bounds_only): every skippable Bounded
     // pushes its bound and every skippable Instances its root fence, flagged, whatever
     // the margin; a sample without the flag took no skip and is exact
@@ -1047,7 +1049,7 @@ __device__ __forceinline__ DeRaw de_run(const DeProgram& P, float3 c, uint32_t m
 }
 // The whole program: exact = false is the reference's de_sample (skippable Bounded
 // branches skipped outside their margin, the sample flagged); exact = true is
-// de_sample_exact (every branch evaluated).
+// de_sample_exact (no margins: every branch that can be the sample evaluated).
 static __device__ __noinline__ DeRaw de_generic(const DeProgram& P, float3 c, bool exact) {
     return de_run(P, c, exact ? SF_EVAL_EXACT : SF_EVAL_FAST, 0, P.n_ops);
 }
@@ -1105,8 +1107,8 @@ __device__ __forceinline__ DeRaw de_raw(const DeProgram& P, float3 p) {
     default: return de_generic(P, p, false);
     }
 }
-// de_sample_exact: the generic program with every Bounded branch evaluated; the
-// specialised forms have no bounds. The path tracers take this whole-program form:
+// de_sample_exact: the generic program with every branch evaluated that can be the
+// sample; the specialised forms have no bounds. The path tracers take this whole-program form:
 // their exact samples (normals, acceptance, refinement) are a small share of their
 // work, and the search's call would raise their register allocation.
 __device__ __forceinline__ DeRaw de_raw_exact(const DeProgram& P, float3 p) {

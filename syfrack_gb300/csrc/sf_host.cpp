@@ -828,8 +828,8 @@ template <class F> void host_parallel(size_t n, size_t grain, F&& f, size_t most
 // speed (100 MB in 0.56 ms, as into pinned memory), and a second pass over the data by
 // host threads cost 5 to 9 ms. What is slow is memory that has never been touched, whose
 // pages the copy then maps one by one (3.8 ms for 100 MB): populate_pages maps them, after
-// the launch and while the device works, without changing what they hold (1.4 ms on 3
-// threads; touching each page with a read and a write took 33 ms, the read mapping the
+// the launch and while the device works, without changing what they hold (2.7 ms on one
+// thread, 1.7, 1.35 and 1.35 on two, three and four, 1.8 on five or six; touching each page with a read and a write took 33 ms, the read mapping the
 // zero page that the write then replaces). Where the kernel does not know the request it
 // is without effect.
 #ifndef MADV_POPULATE_WRITE

@@ -234,7 +234,7 @@ static __device__ __forceinline__ OrbitQuad load_quad(const float2* p) {  // 32-
 
 // One iteration of a pixel's offset d from Z_m = z0 to Z_(m+1) = z1: the new point z, its
 // |z|^2 and the offset's |d|^2. The sums of pairs are packed (each half rounds as a
-// binary32 operation): 40.9 -> 36.7 ms.
+// binary32 operation): 40.9 -> 35.9 ms, with one vote a chunk.
 static __device__ __forceinline__ void pert_step(float2 z0, float2 z1, F2 dc, F2& d, float2& z, float& mag, float& dd) {
     const float2 v = unpack2(d), t = unpack2(fma2(dup2(2.0f), pack2(z0.x, z0.y), d));
     d = add2(pack2(diff_of_products(t.x, v.x, t.y, v.y), sum_of_products(t.x, v.y, t.y, v.x)), dc);

@@ -93,7 +93,8 @@ struct TraceLaunch {
     uint32_t optics;              // 1: the scene has dielectric materials (the optics trace kernel)
     // a single job's form constants: as kernel parameters they are operands from the
     // constant bank, where copies in shared memory took a load or a register each
-    // (64 registers instead of 72 and 119.4 instead of 126.6 ms per 64-spp Mandelbox frame)
+    // (64 registers instead of 72 and 119.4 instead of 126.6 ms per 64-spp Mandelbox frame;
+    // iterations in pairs took it to 68)
     FormParams fp;
 };
 

@@ -284,7 +284,7 @@ class RenderSession:
         w, h = self.cfg.width, self.cfg.height
         acc, aux, color = (np.empty((h, w, 4), np.float32) for _ in range(3))
         depth = np.empty((h, w), np.float32)
-        # the library fills every plane, the mean colour included (pinned staging, host threads)
+        # the library fills every plane, the mean colour included
         planes = sf_film_planes(_fp(acc), _fp(depth), _fp(aux), None, None, None, _fp(color))
         check(self.ctx.lib.sf_session_readback(self.h, C.byref(planes)))
         p = self.progress()
