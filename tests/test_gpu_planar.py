@@ -162,3 +162,25 @@ def test_escape2d_twelve_stripes_off_the_common_loop(gpu_ctx, oracle_mod, family
     d = np.abs(out["traps"].reshape(4, -1).T - ref["traps"])
     assert np.quantile(d, 0.999) <= 0.006
     np.testing.assert_allclose(out["distance"].ravel(), ref["distance"], atol=1e-5)
+
+
+@pytest.mark.parametrize("bailout,term", [(16.0, 7.4e-6), (1e30, 1.4e-5)])
+def test_long_stripe_sums_against_64_bits(gpu_ctx, bailout, term):
+    """The stripe band of interior pixels after 20,000 iterations, in the z^2 loop (double
+    angle) and the unrolled recurrence (a bailout past that loop), against the sum in 64
+    bits over the same binary32 orbit. A term is off by at most `term`, and each addition to
+    a sum of at most n by half of an ulp of n; the band is half of the mean."""
+    n = 20000
+    c = Canvas(width=33, height=17, center=(-0.1, 0.1), zoom=20.0)
+    out = escape2d(gpu_ctx, PlanarFractal(family="Mandelbrot", iterations=n, bailout=bailout), c)
+    assert np.all(out["iterations"] == n)
+    cx, cy = np.ascontiguousarray(canvas_points(c).astype(np.float32).T)
+    x, y, total = np.zeros_like(cx), np.zeros_like(cx), np.zeros(len(cx))
+    for _ in range(n):
+        total += np.sin(12.0 * np.arctan2(y.astype(np.float64), x.astype(np.float64)))
+        m = x * y
+        x, y = (x * x - y * y) + cx, (m + m) + cy
+    assert x.dtype == np.float32
+    err = np.abs(out["traps"][2].ravel() - (0.5 + 0.5 * total / n))
+    print(f"bailout {bailout:g}: stripe band error max {err.max():.3e}, rms {np.sqrt(np.mean(err ** 2)):.3e}")
+    assert err.max() <= 0.5 * term + 0.25 * float(np.spacing(np.float32(n))) + 1e-6
