@@ -322,9 +322,10 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 }
 
 // 2 clamp(x, -l, l) - x of the box fold, bit for bit but for the sign of a zero (the
-// clamped form's zeros are +0, see the trap in de_box_t), in two instructions for three: with t = 2 l - |x| it is the smaller of |x| and |t|, with the
-// sign of x times that of t. (|x| <= l: t rounds to no less than |x|. Past l, t is the
-// fold of |x|, rounded once as the fused form is, and |t| <= |x|.) 0 <= l <= 1e38.
+// clamped form's zeros are +0, see the trap in de_box_t), in two instructions for three:
+// with t = 2 l - |x| it is the smaller of |x| and |t|, with the sign of x times that of t.
+// (|x| <= l: t rounds to no less than |x|. Past l, t is the fold of |x|, rounded once as
+// the fused form is, and |t| <= |x|.) 0 <= l <= 1e38.
 __device__ __forceinline__ float box_fold(float x, float l2) {
     float q;
     asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(q) : "f"(x), "f"(l2 - fabsf(x)));
