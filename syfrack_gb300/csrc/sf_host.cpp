@@ -578,6 +578,35 @@ struct Lowerer {
     }
 };
 
+// DeProgram.run: an op ends its run if a lane may leave its way there (a loop, a bounded
+// branch, a copy search) or if lanes may come to the next op by another (the target of a
+// jump, a leaf's first op).
+void mark_runs(DeProgram& P) {
+    bool ends[SF_MAX_OPS + 1] = {};  // op i ends its run
+    auto joins = [&](uint32_t op) {  // lanes come to `op` by a jump
+        if (op > 0) ends[op - 1] = true;
+    };
+    for (uint32_t i = 0; i < P.n_ops; ++i) {
+        const DeOp& op = P.ops[i];
+        switch (op.code) {
+        case SF_OP_BOUND_FAST: case SF_OP_ITER_BEGIN: case SF_OP_INST_BEGIN:
+            ends[i] = true;
+            joins(op.b + 1);
+            break;
+        case SF_OP_ITER_END: case SF_OP_INST_END:
+            ends[i] = true;
+            joins(op.a + 1);
+            break;
+        default: break;
+        }
+    }
+    for (uint32_t k = 0; k < P.union_leaves; ++k) {
+        joins(P.leaf_begin[k]);
+        joins(P.leaf_end[k]);
+    }
+    for (uint32_t i = P.n_ops; i-- > 0;) P.run[i] = uint8_t(ends[i] || i + 1 == P.n_ops ? 1 : 1 + P.run[i + 1]);
+}
+
 // Largest float x with sqrtf(x) <= b. sqrtf is correctly rounded and monotonic,
 // so |p| > b (the reference's `p.length() > bailout`) is exactly dot(p,p) > T.
 float sqrt_threshold(float b) {
@@ -1023,6 +1052,7 @@ sf_status build_graph(const sf_graph_desc* d, HostGraph& g, DeProgram& P, sf_gra
         }
     }
     P.inst_floats = uint32_t(inst.size());
+    mark_runs(P);
     detect_form(g, P);
     std::memset(&info, 0, sizeof info);
     info.step_scale = g.safety / lip;

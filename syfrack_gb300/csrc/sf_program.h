@@ -98,8 +98,11 @@ struct DeProgram {
     // after the ops, whose offset in shared memory stays that of the plain program.
     uint32_t union_leaves;
     uint8_t leaf_begin[SF_MAX_UNION_LEAVES], leaf_end[SF_MAX_UNION_LEAVES];
+    // run[i]: how many ops from op i on the lanes that stand at i run together: to the next
+    // op that can part them, or to the last one before an op where others may wait.
+    uint8_t run[SF_MAX_OPS + 1];
 };
-static_assert(SF_MAX_OPS <= 255, "leaf ranges are stored as bytes");
+static_assert(SF_MAX_OPS <= 255, "leaf ranges and runs are stored as bytes");
 
 // One area light in device form (GpuLight of uniforms.rs:671-713 with the
 // derived quantities the shading code needs every bounce).

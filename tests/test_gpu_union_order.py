@@ -4,10 +4,11 @@ other branches left out) must give the same sample bit for bit."""
 import numpy as np
 import pytest
 
-from helpers import lcg_points
+from helpers import bounded_bulb, lcg_points
 from syfrack_gb300 import Camera
-from syfrack_gb300.graph import Kind
-from test_union_bound import _Builder, _bulb, _shape
+from syfrack_gb300.graph import Graph, Kind
+from test_gpu_de import kitchen_sink
+from test_union_bound import _Builder, _bulb, _shape, union_world
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +48,31 @@ def test_every_order_gives_the_same_sample(renderer, order, nested):
     p, q = (renderer.primary(g, cam, 120, 90, rule="cone") for g in (base, other))
     for k in ("t", "steps", "normal"):
         np.testing.assert_array_equal(p[k], q[k], err_msg=k)
+
+
+def copies_of_a_bulb(depth):
+    """Copies of a bounded loop, `depth` Instances deep, beside a loop of no iterations."""
+    b = _Builder()
+    d = _bulb(b, (0.0, 0.0, 0.0), 1)
+    for _ in range(depth):
+        d = b.add(Kind("Instances", placements=COPIES, half=[2.5, 2.5, 2.5], margin=0.05), [d])
+    still = b.add(Kind("Iterate", iterations=1, bailout=0.01, body=[b.add(Kind("Abs", x=True, y=True, z=True))]), [0])
+    return b.graph(b.add(Kind("Union"), [d, b.add(Kind("Torus", radius=1.5, tube=0.1), [still])]))
+
+
+GRAPHS = {"one op": lambda: Graph.bundled("sphere"), "kitchen sink": kitchen_sink, "bounded": bounded_bulb,
+          "union": lambda: world((3, 1, 2, 0), True), "nine leaves": union_world, "copies": lambda: copies_of_a_bulb(1),
+          "nested copies": lambda: copies_of_a_bulb(2)}
+
+
+@pytest.mark.parametrize("name", list(GRAPHS))
+def test_lanes_together_and_apart(renderer, name):
+    """Runs of ops between the places where a warp's lanes part and join: the same points
+    beside others of every distance, and with a warp to each, sample for sample."""
+    g = renderer.compile(GRAPHS[name]())
+    pts = np.concatenate([lcg_points(500, 2.5, 17), lcg_points(499, 30.0, 18)])
+    mixed, alone = g.probe(pts[np.random.default_rng(4).permutation(len(pts))]), g.probe(np.repeat(pts, 32, axis=0))
+    order = np.random.default_rng(4).permutation(len(pts))
+    for k in ("distance", "material", "iterations", "traps"):
+        np.testing.assert_array_equal(mixed[k], alone[k][::32][order], err_msg=k)
+        np.testing.assert_array_equal(alone[k][::32], alone[k][31::32], err_msg=k)
