@@ -390,7 +390,7 @@ extern "C" sf_status sf_batch_readback(sf_batch* b, uint32_t job, sf_film_planes
     if (job >= b->jobs.size()) return fail(SF_ERR_INVALID, "job index out of range");
     sf_context* c = b->ctx;
     cudaSetDevice(c->device);
-    CU(film_readback(b->jobs[b->slot[job]].film, *out, c->stream));
+    CU(film_readback(c, b->jobs[b->slot[job]].film, *out, c->stream));
     return SF_OK;
 }
 

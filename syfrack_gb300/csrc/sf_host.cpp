@@ -852,36 +852,48 @@ template <class F> void host_parallel(size_t n, size_t grain, F&& f, size_t most
     for (auto& t : pool) t.join();
 }
 
-// Results go from the device straight into the caller's (pageable) buffers: this
-// platform's copy engine reads and writes host memory through its page tables at link
-// speed (100 MB in 0.56 ms, as into pinned memory), and a second pass over the data by
-// host threads cost 5 to 9 ms. What is slow is memory that has never been touched, whose
-// pages the copy then maps one by one (3.8 ms for 100 MB): populate_pages maps them, after
-// the launch and while the device works, without changing what they hold (2.7 ms on one
-// thread, 1.7, 1.35 and 1.35 on two, three and four, 1.8 on five or six; touching each page with a read and a write took 33 ms, the read mapping the
-// zero page that the write then replaces). Where the kernel does not know the request it
-// is without effect.
+// Results go from the device straight into the caller's (pageable) buffers: this platform's
+// copy engine reads and writes host memory through its page tables at link speed (100 MB in
+// 0.56 ms, as into pinned memory), and a second pass over the data by host threads cost 5 to
+// 9 ms. What is slow is memory that has never been touched, whose pages the copy then maps
+// one by one (3.8 ms for 100 MB): populate_pages maps them, after the launch and while the
+// device works, without changing what they hold (2.7 ms on one thread, 1.7, 1.35 and 1.35 on
+// two, three and four, 1.8 on five or six; touching each page with a read and a write took
+// 33 ms, the read mapping the zero page that the write then replaces). Where the kernel does
+// not know the request it is without effect.
+//
+// Small results go through the context's pinned staging: a copy into pageable memory takes
+// about 10 us more to start, as long as the second pass over 128 KB, so up to that for each
+// copy saved. Film readbacks (four copies) of 1x1 22 us staged and 52 direct, 96x96 (332 KB)
+// 58 and 70, 112x112 (452 KB) 73 and 74, 256x256 300 and 150; tiles (three) of 16x16 38 and
+// 58 us, 112x112 (301 KB) 57 and 58, 128x128 (393 KB) 62 and 57; deep zooms (three) of
+// 192x192 (295 KB) 74 and 78 us, 256x256 (524 KB) 95 and 79.
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
 struct HostOut {
-    void* p;
+    void* to;  // null: not wanted
+    const void* from;
     size_t bytes;
 };
 void populate_pages(std::initializer_list<HostOut> outs) {
     static const size_t page = size_t(std::max<long>(sysconf(_SC_PAGESIZE), 4096));
     for (const HostOut& o : outs) {
-        if (!o.p || !o.bytes) continue;
-        const uintptr_t b = reinterpret_cast<uintptr_t>(o.p) / page;
-        const size_t pages = (reinterpret_cast<uintptr_t>(o.p) + o.bytes + page - 1) / page - b;
+        if (!o.to || !o.bytes) continue;
+        const uintptr_t b = reinterpret_cast<uintptr_t>(o.to) / page;
+        const size_t pages = (reinterpret_cast<uintptr_t>(o.to) + o.bytes + page - 1) / page - b;
         host_parallel(pages, std::max<size_t>((size_t(16) << 20) / page, 1), [&](size_t k, size_t end) {
             madvise(reinterpret_cast<void*>((b + k) * page), (end - k) * page, MADV_POPULATE_WRITE);
         }, 4);
     }
 }
 
-// The context's pinned staging at `bytes` or more (stage_mu held).
+constexpr size_t kStagedEach = size_t(128) << 10;
+
+// The context's pinned staging at `bytes` or more, as much as small results need at least
+// (stage_mu held).
 cudaError_t ensure_stage(sf_context* c, size_t bytes) {
+    bytes = std::max(bytes, 8 * kStagedEach);
     if (c->stage_bytes >= bytes) return cudaSuccess;
     if (c->stage) cudaFreeHost(c->stage);
     c->stage = nullptr;
@@ -889,6 +901,49 @@ cudaError_t ensure_stage(sf_context* c, size_t bytes) {
     cudaError_t e = cudaHostAlloc(&c->stage, bytes, cudaHostAllocDefault);
     if (e == cudaSuccess) c->stage_bytes = bytes;
     return e;
+}
+
+// Copies a call's results to the caller, after the launches on st, and waits for them
+// (stage_mu held, by `lk` or by the caller).
+cudaError_t copy_results(sf_context* c, std::initializer_list<HostOut> outs, cudaStream_t st,
+                         std::unique_lock<std::mutex>* lk = nullptr) {
+    struct Piece {  // of the staging: what neighbours on the device share is one copy
+        const char* from;
+        size_t at, bytes;
+    } pieces[8];
+    size_t n = 0, staged = 0, copies = 0;
+    for (const HostOut& o : outs) {
+        const char* const from = static_cast<const char*>(o.from);
+        if (!o.to || !o.bytes) continue;
+        ++copies;
+        if (std::any_of(pieces, pieces + n, [&](const Piece& p) { return from >= p.from && from < p.from + p.bytes; }))
+            continue;
+        if (n && pieces[n - 1].from + pieces[n - 1].bytes == from) pieces[n - 1].bytes += o.bytes;
+        else pieces[n++] = {from, staged, o.bytes};
+        staged += o.bytes;
+    }
+    cudaError_t e = cudaSuccess;
+    if (staged > copies * kStagedEach) {
+        populate_pages(outs);
+        for (const HostOut& o : outs)
+            if (o.to && o.bytes && e == cudaSuccess) e = cudaMemcpyAsync(o.to, o.from, o.bytes, cudaMemcpyDeviceToHost, st);
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    }
+    if (lk) lk->lock();
+    e = ensure_stage(c, staged);
+    char* const stage = static_cast<char*>(c->stage);
+    for (size_t i = 0; i < n && e == cudaSuccess; ++i)
+        e = cudaMemcpyAsync(stage + pieces[i].at, pieces[i].from, pieces[i].bytes, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    for (const HostOut& o : outs) {
+        if (!o.to || !o.bytes) continue;
+        const char* const from = static_cast<const char*>(o.from);
+        const Piece* p = pieces;
+        while (from < p->from || from >= p->from + p->bytes) ++p;
+        std::memcpy(o.to, stage + p->at + (from - p->from), o.bytes);
+    }
+    return cudaSuccess;
 }
 
 // The context's device scratch at `bytes` or more (stage_mu held), within the budget.
@@ -1406,6 +1461,10 @@ extern "C" sf_status sf_context_create(int device, uint64_t budget, sf_context**
     c->d_stats = static_cast<unsigned long long*>(p);
     c->d_work = reinterpret_cast<uint32_t*>(c->d_stats + SF_STAT_COUNT);
     cudaMemsetAsync(p, 0, SF_STAT_COUNT * sizeof(unsigned long long) + 64 * sizeof(uint32_t), c->stream);
+    // The staging now, so that no call pays for it; small pinned blocks allocated later (a
+    // preview's status word) then find room beside it: previews are created in 0.25 instead of
+    // 0.37 ms and destroyed in 0.08 instead of 0.25. Without it the calls that need it retry.
+    if (ensure_stage(c, 0) != cudaSuccess) cudaGetLastError();
     *out = c;
     return SF_OK;
 }
@@ -1618,10 +1677,7 @@ extern "C" sf_status sf_de_probe(sf_graph* g, const float* xyz, size_t n, sf_de_
         const ProbeArrays io{d_in, d_in + 1, d_in + 2, d_out, d_out + 1, u + 5, u + 6, 3, 7, 1};
         e = sf_launch_de_probe(g->d_prog, io, n, c->stream);
     }
-    populate_pages({{out, n * sizeof(sf_de_sample)}});
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out, d_out, n * sizeof(sf_de_sample), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = copy_results(c, {{out, d_out, n * sizeof(sf_de_sample)}}, c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "sf_de_probe");
     return SF_OK;
 }
@@ -1664,11 +1720,8 @@ static sf_status primary_trace(sf_graph* g, const sf_primary_desc* d, float* t_o
                                dt, ds, dn, rows ? size_t(3) : size_t(1), rows ? size_t(1) : n, c->d_work, c->d_stats};
         e = sf_launch_primary(g->prog.form, g->d_prog, dS, pl, c->stream);
     }
-    populate_pages({{t_out, n * 4}, {steps_out, n * 4}, {normal_out, n * 12}});
-    if (e == cudaSuccess) e = cudaMemcpyAsync(t_out, dt, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(steps_out, ds, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(normal_out, dn, n * 12, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess)
+        e = copy_results(c, {{t_out, dt, n * 4}, {steps_out, ds, n * 4}, {normal_out, dn, n * 12}}, c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "sf_primary_trace");
     return SF_OK;
 }
@@ -2023,23 +2076,15 @@ namespace sfh {
 // (RenderOutput.color); a film without the volume layer split (no fog) has a zero volume
 // contribution: volume and moments are (0, 0, 0, samples) and surface = accum. These
 // planes receive accum and are derived in place by the host threads.
-cudaError_t film_readback(const FilmPlanes& f, const sf_film_planes& out, cudaStream_t st) {
+cudaError_t film_readback(sf_context* c, const FilmPlanes& f, const sf_film_planes& out, cudaStream_t st) {
     const size_t px = size_t(f.width) * f.height;
     const bool split = f.vol != nullptr;
-    populate_pages({{out.accum, px * 16}, {out.depth, px * 4}, {out.aux, px * 16}, {out.volume, px * 16},
-                 {out.moments, px * 16}, {out.surface, px * 16}, {out.color, px * 16}});
-    cudaError_t e = cudaSuccess;
-    auto copy = [&](float* to, const void* from, size_t bytes) {
-        if (to && e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, st);
-    };
-    copy(out.accum, f.accum, px * 16);
-    copy(out.depth, f.depth, px * 4);
-    copy(out.aux, f.aux, px * 16);
-    copy(out.color, f.accum, px * 16);
-    copy(out.volume, split ? f.vol : f.accum, px * 16);
-    copy(out.moments, split ? f.vmom : f.accum, px * 16);
-    copy(out.surface, split ? f.surf : f.accum, px * 16);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    std::unique_lock<std::mutex> lk(c->stage_mu, std::defer_lock);
+    const cudaError_t e = copy_results(c, {{out.accum, f.accum, px * 16}, {out.depth, f.depth, px * 4},
+                                           {out.aux, f.aux, px * 16}, {out.color, f.accum, px * 16},
+                                           {out.volume, split ? f.vol : f.accum, px * 16},
+                                           {out.moments, split ? f.vmom : f.accum, px * 16},
+                                           {out.surface, split ? f.surf : f.accum, px * 16}}, st, &lk);
     if (e != cudaSuccess) return e;
     float* const zero[2] = {split ? nullptr : out.volume, split ? nullptr : out.moments};
     if (!out.color && !zero[0] && !zero[1]) return cudaSuccess;
@@ -2065,7 +2110,7 @@ extern "C" sf_status sf_session_readback(sf_session* s, sf_film_planes* out) {
     if (!s || !out) return fail(SF_ERR_INVALID, "null argument");
     sf_context* c = s->ctx;
     cudaSetDevice(c->device);
-    CU(film_readback(s->film, *out, c->stream));
+    CU(film_readback(c, s->film, *out, c->stream));
     return SF_OK;
 }
 
@@ -2390,11 +2435,7 @@ extern "C" sf_status sf_escape2d(sf_context* c, const sf_planar_desc* f, const s
         e = sf_launch_escape2d(dF, dK, tile.x, tile.y, tile.w, tile.h, sample, dd, dt, di, c->d_stats, dW, 1,
                                F.family == 3 || F.family == 4, c->stream);
     }
-    populate_pages({{dist, n * 4}, {traps, n * 16}, {iters, n * 4}});
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dist, dd, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(traps, dt, n * 16, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(iters, di, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = copy_results(c, {{dist, dd, n * 4}, {traps, dt, n * 16}, {iters, di, n * 4}}, c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "sf_escape2d");
     return SF_OK;
 }
@@ -2507,14 +2548,10 @@ extern "C" sf_status sf_deep_zoom(sf_context* c, const sf_deep_zoom_desc* d, uin
                                  d->bailout, di64, ds64, c->stream);
     }
     const size_t n64 = reference_f64 ? n * 4 : 0;
-    populate_pages({{iters, n * 4}, {smooth, n * 4}, {iters64, n64}, {smooth64, n64}});
-    if (e == cudaSuccess) e = cudaMemcpyAsync(iters, di, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(smooth, ds, n * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess && n64) e = cudaMemcpyAsync(iters64, di64, n64, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess && n64) e = cudaMemcpyAsync(smooth64, ds64, n64, cudaMemcpyDeviceToHost, c->stream);
     unsigned long long after[SF_STAT_COUNT];
-    if (e == cudaSuccess) e = cudaMemcpyAsync(after, c->d_stats, sizeof after, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess)
+        e = copy_results(c, {{iters, di, n * 4}, {smooth, ds, n * 4}, {iters64, di64, n64}, {smooth64, ds64, n64},
+                             {after, c->d_stats, sizeof after}}, c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "sf_deep_zoom");
     if (rebases) *rebases = after[SF_STAT_STEPS] - before[SF_STAT_STEPS];
     return SF_OK;

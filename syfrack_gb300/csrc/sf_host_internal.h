@@ -171,7 +171,7 @@ bool has_hdri(const sf_scene_desc& d);
 sf_status check_launch(uint32_t min_blocks, uint32_t quantum, uint32_t regen, bool small_blocks);
 void planar_dev(const sf_planar_desc& f, PlanarDev& o);
 sf_status planar_check(const sf_planar_desc* f);
-cudaError_t film_readback(const FilmPlanes& f, const sf_film_planes& out, cudaStream_t st);
+cudaError_t film_readback(sf_context* c, const FilmPlanes& f, const sf_film_planes& out, cudaStream_t st);
 // Fog scenes keep the film's volume layer split (volume, moments and surface planes).
 inline bool has_fog(const sf_scene_desc& d) { return d.fog.density > 0.0f; }
 // DevScene.rich of a scene: finish details, a texture, optics (SF_RICH_* bits).

@@ -205,7 +205,7 @@ extern "C" sf_status sf_preview_readback(sf_preview* p, sf_film_planes* out) {
     f.aux = p->out.aux;
     f.width = p->width;
     f.height = p->height;
-    CU(film_readback(f, *out, p->stream));
+    CU(film_readback(p->ctx, f, *out, p->stream));
     return SF_OK;
 }
 

@@ -184,3 +184,13 @@ def test_long_stripe_sums_against_64_bits(gpu_ctx, bailout, term):
     err = np.abs(out["traps"][2].ravel() - (0.5 + 0.5 * total / n))
     print(f"bailout {bailout:g}: stripe band error max {err.max():.3e}, rms {np.sqrt(np.mean(err ** 2)):.3e}")
     assert err.max() <= 0.5 * term + 0.25 * float(np.spacing(np.float32(n))) + 1e-6
+
+
+def test_tiles_around_the_staged_size(gpu_ctx):
+    """Three planes, 24 bytes a pixel: 16,384 go through the pinned staging (3 x 128 KB), 16,385
+    straight to the caller."""
+    f, c = PlanarFractal(family="Julia", iterations=60), Canvas(width=16385, height=1, center=(-0.1, 0.05), zoom=1.5)
+    a, b = escape2d(gpu_ctx, f, c), escape2d(gpu_ctx, f, c, tile=(0, 0, 16384, 1))
+    assert len(np.unique(a["iterations"])) > 10
+    for k in ("iterations", "distance", "traps"):
+        np.testing.assert_array_equal(a[k][..., :16384], b[k], err_msg=k)

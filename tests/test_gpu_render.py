@@ -278,3 +278,41 @@ def test_skippable_bound_film(renderer, oracle_mod, graph):
     hit = ref["depth"] >= 0
     np.testing.assert_array_equal(a.depth[pix[:, 1], pix[:, 0]] >= 0, hit)
     np.testing.assert_allclose(a.depth[pix[:, 1], pix[:, 0]][hit], ref["depth"][hit], rtol=1e-3)
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (64, 128), (64, 129), (160, 120), (200, 130)])
+@pytest.mark.parametrize("fog", [False, True])
+def test_readback_planes_together_and_one_by_one(renderer, w, h, fog):
+    """Planes read through the pinned staging (up to 128 KB for each) or straight into the
+    caller's memory: all seven in one call (36 bytes a pixel, 84 in fog) and each alone (4 or
+    16: 64x128 is 128 KB)."""
+    import ctypes as C
+
+    from helpers import golden_scene
+    from syfrack_gb300._lib import check, sf_film_planes
+
+    scene = golden_scene("mandelbulb", atmosphere={"fog_density": 0.018, "fog_color": [0.8, 0.85, 0.9]} if fog else None)
+    cfg = RenderConfig(w, h, 2, max_bounces=2, max_steps=256, pixel_tolerance=1.0, tile_size=256, samples_per_dispatch=2,
+                       integrator="wavefront")
+    s = RenderSession(renderer, scene, cfg)
+    while not s.step(0):
+        pass
+    names = [f[0] for f in sf_film_planes._fields_]
+
+    def read(wanted):
+        out = {k: np.full((h, w) if k == "depth" else (h, w, 4), -7.0, np.float32) for k in wanted}
+        p = sf_film_planes(*(out[k].ctypes.data_as(C.POINTER(C.c_float)) if k in out else None for k in names))
+        check(s.ctx.lib.sf_session_readback(s.h, C.byref(p)))
+        return out
+
+    every = read(names)
+    for k in names:
+        np.testing.assert_array_equal(read([k])[k], every[k], err_msg=k)
+    n = np.maximum(every["accum"][..., 3:], 1)
+    np.testing.assert_array_equal(every["color"][..., :3], every["accum"][..., :3] / n)
+    assert np.all(every["color"][..., 3] == 1) and np.all(every["accum"][..., 3] == 2)
+    if not fog:
+        assert np.all(every["volume"][..., :3] == 0) and np.all(every["moments"][..., 3] == 2)
+        np.testing.assert_array_equal(every["surface"], every["accum"])
+    s.close()
+
