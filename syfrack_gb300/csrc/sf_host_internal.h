@@ -77,8 +77,8 @@ struct sf_context {
     int refs = 1;
     std::mutex mu;
     std::mutex alloc_mu;  // budget accounting (a server thread allocates too)
-    // pinned staging of a host orbit's upload, and the device scratch of probes, primary
-    // rays, escape time and deep zoom: grown on demand and reused by every call (stage_mu
+    // pinned staging of small results and a host orbit's upload, and the device scratch of
+    // probes, primary rays, escape time and deep zoom: grown on demand and reused by every call (stage_mu
     // guards both)
     void* stage = nullptr;
     size_t stage_bytes = 0;
